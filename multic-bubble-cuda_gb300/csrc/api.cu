@@ -57,6 +57,12 @@ int fail(int code, const char* fmt, ...) {
 // kernel.
 constexpr int kMaxWaves = 16;
 constexpr int kMinCollidePlanes = 8;
+// Default split of a batch: balanced runs of one wave up to this many tile-planes per block,
+// fixed chunks above. 34 uneven FP16 cases of 24..58 cells (34 planes per block) take 123 us
+// per update balanced against 137 to 155 in fixed chunks, 37 of 24..50 cells 94 against 96 to
+// 124; 64 of 32..96 cells (230 planes per block) 842 against 809, because neighbouring columns
+// no longer march in step and share less of L2.
+constexpr int kBatchBalancedPlanes = 64;
 
 size_t pop_bytes(int storage) { return storage == mcb::kStF32 ? 4 : 2; }
 
@@ -225,11 +231,62 @@ struct Solver {
     stream = nullptr;
   }
 
+  // Default chunk of z planes per block, from sweeps on GB300 of every collide kernel. With
+  // kPrime planes' worth of priming per block and W resident blocks in one wave, a launch of N
+  // blocks of zc planes takes about
+  //   (zc + kPrime) (N / W whole waves + a last wave of 0.4 + 0.6 r / k),
+  // where the fullest SM runs r of its k blocks in the last wave: a block alone on its SM
+  // takes 0.6 of the time per plane that one of three does (128x128x256 FP32: 1.85, 2.35 and
+  // 3.1 us per plane with 1, 2 and 3 blocks per SM). The chunk with the least such time runs:
+  //   256^3 BF16 (256 columns, 456 blocks per wave): 37 planes, 3.9 waves, 420 us per update
+  //   against 542 with 256 planes in one wave of 256 blocks; 256^3 relaxed FP16 1044 against
+  //   1324; 200^3 relaxed FP32 40 planes, 475 against 571 with 100; 32^3 FP32 (4 columns)
+  //   one plane per block; 128x128x256 stays at 37 planes (one wave of 448 blocks).
+  // Several cases share one launch, their blocks end at different times and the last wave
+  // blurs: there the whole work over W counts, and half a chunk for the end (32 planes for 64
+  // FP16 cases of 32..96 cells: 810 us, within 0.2 % of the best fixed chunk).
+  int default_chunk(const Group& g, long long wave, int per_sm) const {
+    constexpr double kPrime = 2.0;
+    int nzmax = 1;
+    for (int ci : g.members) nzmax = std::max(nzmax, cases[ci].nz);
+    int best = 1;
+    double best_t = 0;
+    for (int zc = 1; zc <= nzmax; ++zc) {
+      long long n = 0;
+      double work = 0;
+      for (int ci : g.members) {
+        const mcb::CaseDesc& d = cases[ci];
+        const long long m = (d.nz + zc - 1) / zc, cols = 1LL * d.tiles_x * d.tiles_y;
+        n += cols * m;
+        work += cols * (d.nz + kPrime * m);
+      }
+      double t;
+      if (g.members.size() == 1) {
+        const long long whole = n / wave, rest = n % wave, sms = wave / per_sm;
+        const double last = rest ? 0.4 + 0.6 * ((rest + sms - 1) / sms) / per_sm : 0.0;
+        t = (zc + kPrime) * (whole + last);
+      } else {
+        t = work / wave + 0.5 * (zc + kPrime);
+      }
+      if (zc == 1 || t < best_t) {
+        best = zc;
+        best_t = t;
+      }
+    }
+    // Chunks of equal length: the same number of blocks, the last one not shorter.
+    if (g.members.size() == 1) {
+      const int m = (nzmax + best - 1) / best;
+      best = (nzmax + m - 1) / m;
+    }
+    return best;
+  }
+
   // Work decomposition of the cases of one group for its variant and z chunk request:
   //   zchunk_req > 0: fixed chunks of that many planes, one block each;
   //   zchunk_req < 0: balanced ranges, -zchunk_req resident waves of equal-work blocks
   //   per kernel;
-  //   zchunk_req == 0: fixed chunks chosen below.
+  //   zchunk_req == 0: fixed chunks (default_chunk), or one balanced wave for a batch of
+  //   small cases (kBatchBalancedPlanes).
   // A member's own fixed chunk (zc_case > 0) overrides the group's unless it is balanced.
   int build_group(Group& g, int nsm) {
     const mcb::Variant v = mcb::kVariants[g.variant];
@@ -250,28 +307,12 @@ struct Solver {
       return fail(MCB_ERR_CUDA, "no resident blocks for tile variant %d", g.variant);
     int zc = g.zchunk_req;
     if (zc <= 0) {
-      // Default split, from sweeps on GB300: when one case's tile columns fit in one
-      // resident wave of collide blocks, cut every column into the same number of chunks so
-      // that the whole case is one wave whose blocks march neighbouring columns in step
-      // (128x128x256: 37 planes, 2 % faster than 16-plane chunks, 2.4 % faster than
-      // balanced runs at FP32). Otherwise 32-plane chunks (512^3: 13 % faster than balanced
-      // runs, 2.5 % faster than 16). A chunk keeps at least 4 planes: on the 64^3 static
-      // bubble 4-plane chunks (256 blocks) run 20.6 us per update against 25.2 with 8 and
-      // 23.6 with 2 (FP32, relaxed g), 14.6 against 17.6 with 8 (FP16, pair kernel,
-      // equilibrium g).
       const long long wave = 1LL * occ_col * nsm;
-      long long cols = 0;
-      int nzmax = 1;
-      for (int ci : g.members) {
-        cols += static_cast<long long>(cases[ci].tiles_x) * cases[ci].tiles_y;
-        nzmax = std::max(nzmax, cases[ci].nz);
-      }
-      if (g.members.size() == 1 && cols <= wave) {
-        const long long m = std::max<long long>(1, std::min<long long>(wave / cols, nzmax / 4));
-        zc = static_cast<int>((nzmax + m - 1) / m);
-      } else {
-        zc = 32;
-      }
+      const bool own_chunks =
+          std::any_of(g.zc_case.begin(), g.zc_case.end(), [](int c) { return c > 0; });
+      if (g.members.size() > 1 && !own_chunks && g.planes <= kBatchBalancedPlanes * wave)
+        g.balanced = 1;  // one wave of equal runs
+      zc = default_chunk(g, wave, occ_col);
     }
     long long tile0 = 0;
     for (size_t k = 0; k < g.members.size(); ++k) {
@@ -284,7 +325,7 @@ struct Solver {
       if (tile0 > 0x7fffffffLL) return fail(MCB_ERR_INVALID, "too many tiles (%lld)", tile0);
     }
     g.ntiles = static_cast<int>(tile0);
-    g.zchunk = g.balanced ? g.zchunk_req : zc;
+    g.zchunk = g.balanced ? std::min(g.zchunk_req, -1) : zc;
     g.phi_balanced = 0;
     if (g.balanced) {
       const int waves = -g.zchunk;

@@ -279,6 +279,34 @@ __device__ __forceinline__ void for_each_segment(const StepArgs& a, Body&& body,
   }
 }
 
+// The tile of this block when the launch holds one case in fixed chunks (StepArgs::single).
+// Everything here comes from the kernel's parameters and the block index, so the compiler
+// keeps it, and what follows from it, in uniform registers.
+template <int BX, int BY>
+__device__ __forceinline__ Tile single_tile(const StepArgs& a) {
+  const CaseDesc& c = a.one;
+  Tile t;
+  t.ci = 0;
+  t.nx = c.nx;
+  t.ny = c.ny;
+  t.nz = c.nz;
+  t.bc = c.bc;
+  t.zb = static_cast<int>(blockIdx.z) * c.zchunk;
+  t.ze = min(t.nz, t.zb + c.zchunk);
+  t.xt = static_cast<int>(blockIdx.x) * BX;
+  t.yt = static_cast<int>(blockIdx.y) * BY;
+  t.ncell = c.ncell;
+  t.cell_off = 0;
+  t.f_off = 0;
+  t.g_off = 0;
+  t.fn = c.fn;
+  t.fgx = c.fgx;
+  t.fpx = c.fpx;
+  t.fpy = c.fpy;
+  t.fxb = c.fxb;
+  return t;
+}
+
 // Register budgets, the largest warp counts per SM that compile without spills: 24 for
 // k_collide (80 registers); for k_phi, 32 with 32-bit storage (64 registers) and 24 with
 // the 16-bit decode (80 registers). Both kernels wait on loads, so resident warps hide
@@ -1530,7 +1558,7 @@ const void* collide_kernel(int variant, dim3* block) {
       // two cells per thread (the instance without the reference-mode shell; launches pick
       // by StepArgs::has_ref)
       *block = dim3(kPairTX, kPairBY);
-      return pair_kernel<S>(variant, false, GM);
+      return pair_kernel<S>(variant, false, GM, false);
     default: return nullptr;
   }
 }
@@ -1573,11 +1601,11 @@ const void* collide_kernel_gm(int variant, int gmode, dim3* block) {
   }
 }
 
-inline cudaError_t launch_on(const void* fn, int grid, dim3 block, const StepArgs& a,
+inline cudaError_t launch_on(const void* fn, dim3 grid, dim3 block, const StepArgs& a,
                              cudaStream_t s, int dyn_smem = 0) {
-  if (!fn || grid <= 0) return cudaErrorInvalidValue;
+  if (!fn || grid.x == 0) return cudaErrorInvalidValue;
   void* args[] = {const_cast<StepArgs*>(&a)};
-  return cudaLaunchKernel(fn, dim3(grid), block, args, static_cast<size_t>(dyn_smem), s);
+  return cudaLaunchKernel(fn, grid, block, args, static_cast<size_t>(dyn_smem), s);
 }
 
 template <class S>
@@ -1662,7 +1690,9 @@ cudaError_t init_storage(const InitArgs& a, int nx, int ny, int nz, cudaStream_t
     if (variant == kTmaVariant)                                                            \
       return gmode == kGEquil ? launch_collide_tma<S>(a, tmap, s) : cudaErrorInvalidValue; \
     if (is_pair_variant(variant))                                                          \
-      return launch_on(pair_kernel<S>(variant, a.has_ref != 0, gmode), a.grid_collide,     \
+      return launch_on(pair_kernel<S>(variant, a.has_ref != 0, gmode, a.single != 0),      \
+                       a.single ? dim3(a.one.tiles_x, a.one.tiles_y, a.one.tiles_z)        \
+                                : dim3(a.grid_collide),                                    \
                        dim3(kPairTX, kPairBY), a, s, pair_dyn_smem<S>(gmode));             \
     if (a.qf == kQ27 || a.ratio || a.wide)                                                 \
       return launch_on(collide27_kernel<S>(gmode, a.qf, a.ratio != 0, a.wide != 0),        \

@@ -237,11 +237,14 @@ __host__ __device__ constexpr int pair_bgk_smem() {
 // kRef: some case of the launch is in reference mode (frozen shell); the shell handling is
 // compiled only into that instance, which also runs the other modes.
 // kL2: prefetch into L2 the f rows of plane z + 2 while plane z collides.
+// kOne: the launch holds one case in fixed chunks, described by the kernel's parameters: the
+// per-plane bases and bounds then come from uniform registers and constants (508 warp
+// instructions per 32 cells against 532 at FP16, 110.3 us against 112.7 on 128x128x256).
 // GM: how g crosses the update (kGEquil: pushed equilibrium populations, nothing stored;
 // kGPop: stored at full relaxation; kGBgk: stored, pulled and relaxed with tau_g != 1). The
 // stored forms run periodic and wall modes only (no reference shell) and need 18 * cells
 // below 2^31 (checked on the host).
-template <class S, int BY, bool kRef, bool kL2, int GM>
+template <class S, int BY, bool kRef, bool kL2, int GM, bool kOne>
 __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Tile& t) {
   constexpr bool EQ = GM == kGEquil;
   constexpr bool BGK = GM == kGBgk;
@@ -276,9 +279,12 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
   const bool active = x0 < nx && y < ny;  // nx is even: x0 + 1 < nx with x0
 
   const CaseDesc* cd = a.cases + t.ci;
-  const float omega = __ldg(&cd->omega), omega_g = __ldg(&cd->omega_g);
-  const float sigma = __ldg(&cd->sigma), sharp_c = __ldg(&cd->sharp_c);
-  const float gravity = __ldg(&cd->gravity), phi_mean = __ldg(&cd->phi_mean);
+  const float omega = kOne ? a.one.omega : __ldg(&cd->omega);
+  const float omega_g = kOne ? a.one.omega_g : __ldg(&cd->omega_g);
+  const float sigma = kOne ? a.one.sigma : __ldg(&cd->sigma);
+  const float sharp_c = kOne ? a.one.sharp_c : __ldg(&cd->sharp_c);
+  const float gravity = kOne ? a.one.gravity : __ldg(&cd->gravity);
+  const float phi_mean = __ldg(&cd->phi_mean);  // from the table: new fields change it
 
   const int* __restrict__ pcur = a.p_cur + t.cell_off;
   int* __restrict__ pnext = a.p_next + t.cell_off;
@@ -963,11 +969,15 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
   for (int q = max(t.ze - 2, t.zb - 1); q <= t.ze; ++q) flush(q);
 }
 
-template <class S, int BY, bool kRef, int kMinBlocks, bool kL2, int GM>
+template <class S, int BY, bool kRef, int kMinBlocks, bool kL2, int GM, bool kOne>
 __global__ void __launch_bounds__(kPairTX * BY, kMinBlocks)
-    k_collide_pair(const StepArgs a) {
+    k_collide_pair(const __grid_constant__ StepArgs a) {
+  if constexpr (kOne) {
+    collide_pair_segment<S, BY, kRef, kL2, GM, true>(a, single_tile<2 * kPairTX, BY>(a));
+    return;
+  }
   for_each_segment<2 * kPairTX, BY, true>(
-      a, [&](const Tile& t) { collide_pair_segment<S, BY, kRef, kL2, GM>(a, t); },
+      a, [&](const Tile& t) { collide_pair_segment<S, BY, kRef, kL2, GM, false>(a, t); },
       a.balanced != 0);
 }
 
@@ -976,21 +986,27 @@ __global__ void __launch_bounds__(kPairTX * BY, kMinBlocks)
 // independent work per warp; two blocks per SM measured 12 % slower at FP16 storage and 26 %
 // at FP32, four blocks at 128 registers 6 % and 18 %). Variant 6: the same with an L2
 // prefetch of the f rows of the plane after next.
-template <class S, int GM>
+template <class S, int GM, bool kOne>
 const void* pair_kernel_gm(int variant, bool with_ref) {
   if constexpr (GM != kGEquil) {
     // stored g: periodic and wall modes only (the host sees to it)
     // relaxed FP32 g: its staged planes leave room for two blocks per SM
     constexpr int MB = (GM == kGBgk && !S::kDev) ? 2 : 3;
     return variant == kPairVariant
-               ? reinterpret_cast<const void*>(k_collide_pair<S, kPairBY, false, MB, false, GM>)
-               : reinterpret_cast<const void*>(k_collide_pair<S, kPairBY, false, MB, true, GM>);
+               ? reinterpret_cast<const void*>(
+                     k_collide_pair<S, kPairBY, false, MB, false, GM, kOne>)
+               : reinterpret_cast<const void*>(
+                     k_collide_pair<S, kPairBY, false, MB, true, GM, kOne>);
   } else if (variant == kPairVariant) {
-    return with_ref ? reinterpret_cast<const void*>(k_collide_pair<S, kPairBY, true, 3, false, GM>)
-                    : reinterpret_cast<const void*>(k_collide_pair<S, kPairBY, false, 3, false, GM>);
+    return with_ref ? reinterpret_cast<const void*>(
+                          k_collide_pair<S, kPairBY, true, 3, false, GM, kOne>)
+                    : reinterpret_cast<const void*>(
+                          k_collide_pair<S, kPairBY, false, 3, false, GM, kOne>);
   } else {
-    return with_ref ? reinterpret_cast<const void*>(k_collide_pair<S, kPairBY, true, 3, true, GM>)
-                    : reinterpret_cast<const void*>(k_collide_pair<S, kPairBY, false, 3, true, GM>);
+    return with_ref ? reinterpret_cast<const void*>(
+                          k_collide_pair<S, kPairBY, true, 3, true, GM, kOne>)
+                    : reinterpret_cast<const void*>(
+                          k_collide_pair<S, kPairBY, false, 3, true, GM, kOne>);
   }
 }
 
@@ -1000,12 +1016,17 @@ int pair_dyn_smem(int gmode) {
   return gmode == kGBgk ? pair_bgk_smem<S>() : 0;
 }
 
+// single: the launch holds one case in fixed chunks (StepArgs::single; not relaxed g).
 template <class S>
-const void* pair_kernel(int variant, bool with_ref, int gmode) {
+const void* pair_kernel(int variant, bool with_ref, int gmode, bool single) {
   switch (gmode) {
-    case kGEquil: return pair_kernel_gm<S, kGEquil>(variant, with_ref);
-    case kGBgk: return pair_kernel_gm<S, kGBgk>(variant, with_ref);
-    case kGPop: return pair_kernel_gm<S, kGPop>(variant, with_ref);
+    case kGEquil:
+      return single ? pair_kernel_gm<S, kGEquil, true>(variant, with_ref)
+                    : pair_kernel_gm<S, kGEquil, false>(variant, with_ref);
+    case kGPop:
+      return single ? pair_kernel_gm<S, kGPop, true>(variant, with_ref)
+                    : pair_kernel_gm<S, kGPop, false>(variant, with_ref);
+    case kGBgk: return single ? nullptr : pair_kernel_gm<S, kGBgk, false>(variant, with_ref);
     default: return nullptr;
   }
 }

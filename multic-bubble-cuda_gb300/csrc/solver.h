@@ -61,6 +61,13 @@ struct CaseDesc {
 //     so every block has the same work and G is a whole number of resident waves.
 struct StepArgs {
   const CaseDesc* cases;
+  // One case in fixed chunks: its description, here in the kernel's parameters, and a grid of
+  // (tiles_x, tiles_y, tiles_z) blocks (single = 1; the pair kernel, g not relaxed).
+  // Otherwise cases and the flat grid hold. All of it but phi_mean (read from cases: new
+  // fields change it and a captured graph keeps its parameters) stays as it is while the
+  // tiles stay.
+  CaseDesc one;
+  int single;
   int ncases;
   int ntiles;
   int balanced;

@@ -165,6 +165,8 @@ struct Solver {
     int ntiles = 0, zchunk = 16, balanced = 1, phi_balanced = 0, planes = 0;
     int grid_phi = 0, grid_collide = 0;
     int table = 0;  // first entry of the group's case table in d_gcases
+    int has_ref = 0, single = 0;  // StepArgs of the same names
+    int chain = 0, smem = 0;
   };
   std::vector<Group> groups;
   bool grouped = false;  // groups set by the batch autotuner (else one group, rebuilt)
@@ -243,8 +245,8 @@ struct Solver {
   //   1324; 200^3 relaxed FP32 40 planes, 475 against 571 with 100; 32^3 FP32 (4 columns)
   //   one plane per block; 128x128x256 stays at 37 planes (one wave of 448 blocks).
   // Several cases share one launch, their blocks end at different times and the last wave
-  // blurs: there the whole work over W counts, and half a chunk for the end (32 planes for 64
-  // FP16 cases of 32..96 cells: 810 us, within 0.2 % of the best fixed chunk).
+  // blurs: there the whole work over W counts, and a chunk for the end (64 FP16 cases of 32..96
+  // cells: 24 planes, 809 us, the best of 4 to 96; 32 planes 810, 52 planes 826).
   int default_chunk(const Group& g, long long wave, int per_sm) const {
     constexpr double kPrime = 3.0;
     int nzmax = 1;
@@ -258,16 +260,18 @@ struct Solver {
         n += cols * m;
         work += cols * (d.nz + kPrime * m);
       }
-      if (g.members.size() > 1) return work / wave + 0.5 * (zc + kPrime);
+      if (g.members.size() > 1) return work / wave + (zc + kPrime);
       const long long whole = n / wave, rest = n % wave, sms = wave / per_sm;
       const double last = rest ? 0.4 + 0.6 * ((rest + sms - 1) / sms) / per_sm : 0.0;
       return (zc + kPrime) * (whole + last);
     };
-    // The longest chunk within 1 % of the least time (fewer primed planes).
+    // The longest chunk within 1 % of the least time (fewer primed planes); for several cases
+    // the chunk of least time itself.
     double least = time_of(1);
     for (int zc = 2; zc <= nzmax; ++zc) least = std::min(least, time_of(zc));
     int best = nzmax;
-    while (time_of(best) > 1.01 * least) --best;
+    const double slack = g.members.size() > 1 ? 1.0 : 1.01;
+    while (time_of(best) > slack * least) --best;
     // Chunks of equal length: the same number of blocks, the last one not shorter.
     if (g.members.size() == 1) {
       const int m = (nzmax + best - 1) / best;
@@ -339,6 +343,38 @@ struct Solver {
       if (g.phi_balanced)
         g.grid_phi = static_cast<int>(std::min<long long>(g.planes, 1LL * occ_phi * nsm));
     }
+    g.has_ref = 0;
+    for (int ci : g.members) g.has_ref = g.has_ref || cases[ci].bc == mcb::kBcRef;
+    // One case in fixed chunks goes by the kernel's parameters where the pair kernel runs
+    // (the y and z limits of a grid hold every lattice: at most 65535 cells per axis). 128 x
+    // 128 x 256: 121.5 us against 123.0 at FP32, 110.3 against 112.7 at FP16; relaxed g stays
+    // with the table (FP16 268 us against 264).
+    g.single = cases.size() == 1 && !g.balanced && mcb::is_pair_variant(g.variant) &&
+               gmode != mcb::kGBgk;
+    return chain_of(g, nsm, occ_col);
+  }
+
+  // Whether a group's collide kernel is chained to the one before it (it may start under that
+  // one's last blocks), and the shared memory that goes with it. Chained blocks take whatever
+  // slots are free while the kernel before them runs: a grid that leaves free a good part of
+  // the slots then crowds on some SMs (64^3 relaxed FP32, 256 blocks on 456 slots: 25.8 us
+  // against 20.8). So a grid below one wave is limited, by its shared memory, to the blocks
+  // per SM that it needs anyway; then no SM holds more than the even spread's most. us per
+  // update, chained against not: 32^3 FP32 5.65 / 6.98, 64^3 FP16 12.6 / 14.1, 64^3 relaxed
+  // FP32 19.7 / 20.8, 80^3 FP32 24.3 / 26.1, 96^3 FP32 33.1 / 35.5, 97x75x61 25.7 / 27.5,
+  // 128x128x256 FP32 120.4 / 121.9, 256^3 BF16 413 / 416. The pair kernel with stored g loses
+  // (128x128x256 165 us against 160) and is not chained, nor is a batch in fixed chunks (64
+  // FP16 cases of 32..96 cells: 849 us against 835).
+  int chain_of(Group& g, int nsm, int occ_col) {
+    g.chain = g.smem = 0;
+    if (!push || (mcb::is_pair_variant(g.variant) && gmode != mcb::kGEquil) ||
+        (g.members.size() > 1 && !g.balanced))
+      return MCB_OK;
+    const int per_sm = (g.grid_collide + nsm - 1) / nsm;
+    if (per_sm < occ_col)
+      MCB_CU(mcb::residency_smem(storage, g.variant, gmode, qf, ratio, wide, g.has_ref, g.single,
+                                 per_sm, &g.smem));
+    g.chain = per_sm >= occ_col || g.smem > 0;
     return MCB_OK;
   }
 
@@ -720,13 +756,10 @@ struct Solver {
     mcb::StepArgs a{};
     a.cases = d_gcases + gr.table;
     a.ncases = static_cast<int>(gr.members.size());
-    for (int ci : gr.members) a.has_ref = a.has_ref || cases[ci].bc == mcb::kBcRef;
-    // One case in fixed chunks goes by the kernel's parameters where the pair kernel runs
-    // (the y and z limits of a grid hold every lattice: at most 65535 cells per axis). 128 x
-    // 128 x 256: 121.5 us against 123.0 at FP32, 110.3 against 112.7 at FP16; relaxed g stays
-    // with the table (FP16 268 us against 264).
-    a.single = cases.size() == 1 && !gr.balanced && mcb::is_pair_variant(gr.variant) &&
-               gmode != mcb::kGBgk;
+    a.has_ref = gr.has_ref;
+    a.chain = gr.chain;
+    a.smem = gr.smem;
+    a.single = gr.single;
     if (a.single) a.one = cases[0];
     a.ntiles = gr.ntiles;
     a.balanced = gr.balanced;

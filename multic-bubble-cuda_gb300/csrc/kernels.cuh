@@ -181,6 +181,15 @@ __device__ __forceinline__ void l2_prefetch(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
+// Programmatic dependent launch of the collide kernels: a block lets the next update's kernel
+// be launched as soon as every block of this one has started, and waits for the previous
+// kernel (complete, its writes visible) before its first access to the lattice. The launch
+// and the set-up of the offsets then run under the previous update's last blocks.
+__device__ __forceinline__ void grid_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // L2 prefetch of one plane of a BX x BY tile in narr arrays: the first and the last
 // element of every row, which covers each row's one or two 128-byte lines. A later update
 // loop iteration then finds these populations in L2. That keeps DRAM busy regardless of
@@ -923,6 +932,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
   // Normals one plane ahead: each plane takes one barrier, after which the normals of
   // plane z+2 go into the fourth ring slot while the collision of plane z reads planes
   // z-1 .. z+1.
+  if constexpr (!kTma) grid_wait();
   // Prologue: phi planes zb-2 .. zb+2, normals zb-1 .. zb+1.
   for (int zpl = t.zb - 2; zpl <= t.zb + 2; ++zpl) {
     issue(zpl);
@@ -1347,6 +1357,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
 template <class S, int GM, int BX, int BY>
 __global__ void __launch_bounds__(BX * BY, kCollideWarpsPerSM * 32 / (BX * BY))
     k_collide(const StepArgs a) {
+  grid_trigger();
   for_each_segment<BX, BY, true>(a,
                                  [&](const Tile& t) { collide_segment<S, GM, BX, BY>(a, t); }, a.balanced != 0);
 }
@@ -1354,6 +1365,7 @@ __global__ void __launch_bounds__(BX * BY, kCollideWarpsPerSM * 32 / (BX * BY))
 // Cases of 2^31 / 19 cells or more: 64-bit f offsets, 32x8 tiles.
 template <class S, int GM>
 __global__ void __launch_bounds__(256, kCollideWarpsPerSM / 8) k_collide_wide(const StepArgs a) {
+  grid_trigger();
   for_each_segment<32, 8, true>(
       a, [&](const Tile& t) { collide_segment<S, GM, 32, 8, false, kQ, false, true>(a, t); }, a.balanced != 0);
 }
@@ -1391,6 +1403,7 @@ constexpr int collide27_blocks() {
 template <class S, int GM, bool kWide>
 __global__ void __launch_bounds__(256, collide27_blocks<S, GM, kWide>())
     k_collide27(const StepArgs a) {
+  grid_trigger();
   for_each_segment<32, 8, true>(
       a, [&](const Tile& t) { collide_segment<S, GM, 32, 8, false, kQ27, false, kWide>(a, t); }, a.balanced != 0);
 }
@@ -1399,6 +1412,7 @@ __global__ void __launch_bounds__(256, collide27_blocks<S, GM, kWide>())
 template <class S, int GM, int QF, bool kWide>
 __global__ void __launch_bounds__(256, QF == kQ27 ? 2 : kCollideWarpsPerSM / 8)
     k_collide_ratio(const StepArgs a) {
+  grid_trigger();
   for_each_segment<32, 8, true>(
       a, [&](const Tile& t) { collide_segment<S, GM, 32, 8, false, QF, true, kWide>(a, t); }, a.balanced != 0);
 }
@@ -1601,11 +1615,31 @@ const void* collide_kernel_gm(int variant, int gmode, dim3* block) {
   }
 }
 
-inline cudaError_t launch_on(const void* fn, dim3 grid, dim3 block, const StepArgs& a,
-                             cudaStream_t s, int dyn_smem = 0) {
+// Launches a collide kernel; with a.chain it may start under the end of the kernel before it
+// in the stream (programmatic stream serialisation; the kernel calls grid_wait). Captured
+// graphs keep it as programmatic edges.
+inline cudaError_t launch_collide_fn(const void* fn, dim3 grid, dim3 block, const StepArgs& a,
+                                  cudaStream_t s, int dyn_smem) {
   if (!fn || grid.x == 0) return cudaErrorInvalidValue;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = static_cast<size_t>(dyn_smem);
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = a.chain ? 1 : 0;
   void* args[] = {const_cast<StepArgs*>(&a)};
-  return cudaLaunchKernel(fn, grid, block, args, static_cast<size_t>(dyn_smem), s);
+  return cudaLaunchKernelExC(&c, fn, args);
+}
+
+inline cudaError_t launch_on(const void* fn, int grid, dim3 block, const StepArgs& a,
+                             cudaStream_t s) {
+  if (!fn || grid <= 0) return cudaErrorInvalidValue;
+  void* args[] = {const_cast<StepArgs*>(&a)};
+  return cudaLaunchKernel(fn, dim3(grid), block, args, 0, s);
 }
 
 template <class S>
@@ -1622,6 +1656,21 @@ template <class S>
 cudaError_t prepare_tma_kernel() {
   return cudaFuncSetAttribute(k_collide_tma<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               TmaBox<typename S::FT>::kSmem);
+}
+
+// Opts a kernel in to the largest dynamic shared memory a block of it may have: one value for
+// every caller, so that no handle lowers what another one needs.
+inline cudaError_t opt_in_smem(const void* fn, int* largest = nullptr) {
+  cudaFuncAttributes at;
+  int dev = 0, block_max = 0;
+  cudaError_t e = cudaFuncGetAttributes(&at, fn);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&block_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e != cudaSuccess) return e;
+  const int most = block_max - static_cast<int>(at.sharedSizeBytes);
+  if (largest) *largest = most;
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
 }
 
 // Resident blocks per SM of the phi and collide kernels of a variant.
@@ -1660,7 +1709,7 @@ cudaError_t occupancy_of(int variant, int gmode, int qf, int ratio, int wide, in
     // shared memory per block is set here.
     dyn = pair_dyn_smem<S>(gmode);
     if (dyn > 0) {
-      e = cudaFuncSetAttribute(fc, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
+      e = opt_in_smem(fc);
       if (e != cudaSuccess) return e;
     }
   }
@@ -1677,6 +1726,52 @@ cudaError_t init_storage(const InitArgs& a, int nx, int ny, int nz, cudaStream_t
   return cudaGetLastError();
 }
 
+// The collide kernel of a launch, its block and the dynamic shared memory that it needs
+// (every form but the TMA one).
+template <class S>
+const void* collide_fn(int variant, int gmode, int qf, bool ratio, bool wide, bool has_ref,
+                       bool single, dim3* block, int* dyn) {
+  *dyn = 0;
+  if (is_pair_variant(variant)) {
+    *block = dim3(kPairTX, kPairBY);
+    *dyn = pair_dyn_smem<S>(gmode);
+    return pair_kernel<S>(variant, has_ref, gmode, single);
+  }
+  if (qf == kQ27 || ratio || wide) {
+    *block = dim3(32, 8);
+    return collide27_kernel<S>(gmode, qf, ratio, wide);
+  }
+  return collide_kernel_gm<S>(variant, gmode, block);
+}
+
+// Dynamic shared memory that keeps a launch of that kernel to per_sm blocks per SM (0: what
+// the kernel needs already does, or it cannot be met), and the kernel's opt-in for it.
+template <class S>
+cudaError_t residency_smem_of(int variant, int gmode, int qf, int ratio, int wide, int has_ref,
+                              int single, int per_sm, int* bytes) {
+  *bytes = 0;
+  if (variant == kTmaVariant) return cudaSuccess;
+  dim3 block;
+  int dyn = 0, dev = 0, sm_total = 0, reserved = 0, largest = 0;
+  const void* fn = collide_fn<S>(variant, gmode, qf, ratio != 0, wide != 0, has_ref != 0,
+                                 single != 0, &block, &dyn);
+  if (!fn) return cudaErrorInvalidValue;
+  cudaFuncAttributes at;
+  cudaError_t e = cudaFuncGetAttributes(&at, fn);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&sm_total, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+  if (e == cudaSuccess)
+    e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+  if (e == cudaSuccess) e = opt_in_smem(fn, &largest);
+  if (e != cudaSuccess) return e;
+  // Past a (per_sm + 1)-th of the SM, in whole kilobytes.
+  const int fixed = static_cast<int>(at.sharedSizeBytes);
+  const int want = (sm_total / (per_sm + 1) - reserved - fixed) / 1024 * 1024 + 1024;
+  if (want > dyn && want <= largest) *bytes = want;
+  return cudaSuccess;
+}
+
 // One storage format per translation unit, so the formats compile in parallel.
 #define MCB_STORAGE_LAUNCHERS(S, suffix)                                                   \
   cudaError_t launch_phi_##suffix(int variant, int gmode, const StepArgs& a,               \
@@ -1689,17 +1784,18 @@ cudaError_t init_storage(const InitArgs& a, int nx, int ny, int nz, cudaStream_t
                                       const void* tmap, cudaStream_t s) {                  \
     if (variant == kTmaVariant)                                                            \
       return gmode == kGEquil ? launch_collide_tma<S>(a, tmap, s) : cudaErrorInvalidValue; \
-    if (is_pair_variant(variant))                                                          \
-      return launch_on(pair_kernel<S>(variant, a.has_ref != 0, gmode, a.single != 0),      \
-                       a.single ? dim3(a.one.tiles_x, a.one.tiles_y, a.one.tiles_z)        \
-                                : dim3(a.grid_collide),                                    \
-                       dim3(kPairTX, kPairBY), a, s, pair_dyn_smem<S>(gmode));             \
-    if (a.qf == kQ27 || a.ratio || a.wide)                                                 \
-      return launch_on(collide27_kernel<S>(gmode, a.qf, a.ratio != 0, a.wide != 0),        \
-                       a.grid_collide, dim3(32, 8), a, s);                                 \
     dim3 block;                                                                            \
-    const void* fn = collide_kernel_gm<S>(variant, gmode, &block);                         \
-    return launch_on(fn, a.grid_collide, block, a, s);                                     \
+    int dyn = 0;                                                                           \
+    const void* fn = collide_fn<S>(variant, gmode, a.qf, a.ratio != 0, a.wide != 0,        \
+                                   a.has_ref != 0, a.single != 0, &block, &dyn);           \
+    const dim3 grid = a.single ? dim3(a.one.tiles_x, a.one.tiles_y, a.one.tiles_z)         \
+                               : dim3(a.grid_collide);                                     \
+    return launch_collide_fn(fn, grid, block, a, s, a.smem > dyn ? a.smem : dyn);          \
+  }                                                                                        \
+  cudaError_t residency_smem_##suffix(int variant, int gmode, int qf, int ratio, int wide, \
+                                      int has_ref, int single, int per_sm, int* bytes) {   \
+    return residency_smem_of<S>(variant, gmode, qf, ratio, wide, has_ref, single, per_sm,  \
+                                bytes);                                                    \
   }                                                                                        \
   cudaError_t prepare_tma_##suffix() { return prepare_tma_kernel<S>(); }                   \
   size_t tma_smem_##suffix() { return TmaBox<typename S::FT>::kSmem; }                     \

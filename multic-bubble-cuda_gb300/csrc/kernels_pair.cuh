@@ -581,6 +581,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
     }
   };
 
+  grid_wait();
   // Prologue: phi planes zb-2 .. zb+2, normals zb-1 .. zb+1.
   for (int zpl = t.zb - 2; zpl <= t.zb + 2; ++zpl) {
     issue(zpl);
@@ -972,6 +973,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
 template <class S, int BY, bool kRef, int kMinBlocks, bool kL2, int GM, bool kOne>
 __global__ void __launch_bounds__(kPairTX * BY, kMinBlocks)
     k_collide_pair(const __grid_constant__ StepArgs a) {
+  grid_trigger();
   if constexpr (kOne) {
     collide_pair_segment<S, BY, kRef, kL2, GM, true>(a, single_tile<2 * kPairTX, BY>(a));
     return;

@@ -1,5 +1,6 @@
-"""The default work split: it covers every plane once whatever the lattice, so the fields do not
-depend on it (bit for bit), and a chunk never exceeds the lattice."""
+"""The default work split and the chained launches that go with it: every plane is covered once
+whatever the lattice, and an update sees the whole of the one before it, so the fields depend
+neither on the split nor on graph replay (bit for bit)."""
 import numpy as np
 import pytest
 
@@ -7,11 +8,13 @@ import mcb
 
 pytestmark = pytest.mark.gpu
 
-# one tile column, ragged columns, one wave, several waves, fewer planes than a chunk
-LATTICES = [(8, 8, 4), (32, 32, 32), (34, 9, 33), (97, 75, 61), (128, 100, 37), (256, 256, 24)]
+# one tile column, ragged columns, grids of one, two and three blocks per SM, several waves,
+# fewer planes than a chunk
+LATTICES = [(8, 8, 4), (32, 32, 32), (34, 9, 33), (64, 64, 64), (97, 75, 61), (128, 100, 37),
+            (256, 256, 24)]
 
 
-def _run(cfg, steps=5):
+def _run(cfg, steps=40):
     d = (cfg.nx, cfg.ny, cfg.nz)
     phi = mcb.fill_phi_bubbles(*d, cfg.bc, 4.0, [(d[0] * 0.47, d[1] * 0.52, d[2] * 0.4, 5.0)])
     with mcb.Solver(cfg) as s:
@@ -27,9 +30,9 @@ def test_default_split_gives_the_fields_of_any_split(dims, tau_g):
               sharp_c=0.0)
     (_, zc), phi, ux = _run(mcb.default_config(**kw))
     assert 1 <= zc <= dims[2]
-    for other in (dims[2], 3, -1):
-        _, phi2, ux2 = _run(mcb.default_config(zchunk=other, **kw))
-        assert np.array_equal(phi, phi2) and np.array_equal(ux, ux2), other
+    for other, graph in ((dims[2], 1), (3, 1), (-1, 1), (0, 0)):
+        _, phi2, ux2 = _run(mcb.default_config(zchunk=other, use_graph=graph, **kw))
+        assert np.array_equal(phi, phi2) and np.array_equal(ux, ux2), (other, graph)
 
 
 def test_small_batch_runs_balanced_and_keeps_the_fields():

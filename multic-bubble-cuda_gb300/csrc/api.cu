@@ -673,8 +673,11 @@ struct Solver {
     return MCB_OK;
   }
 
-  // Error flag of the kernels' bounded waits; read at every synchronisation point.
+  // Error flag of the kernels' bounded waits; read at every synchronisation point. Only the
+  // TMA collide waits, so no other handle pays for the read-back (a blocking copy: 8 updates
+  // of 32^3 cells with five fields read took 172 us with it, 117 without).
   int check_err() {
+    if (!padded) return MCB_OK;
     int h = 0;
     MCB_CU(cudaMemcpy(&h, err, sizeof h, cudaMemcpyDeviceToHost));
     if (h != 0) {

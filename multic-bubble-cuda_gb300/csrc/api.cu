@@ -288,7 +288,7 @@ struct Solver {
   //   small cases (kBatchBalancedPlanes).
   // A member's own fixed chunk (zc_case > 0) overrides the group's unless it is balanced.
   int build_group(Group& g, int nsm) {
-    const mcb::Variant v = mcb::kVariants[g.variant];
+    const mcb::Variant v = mcb::tile_of(g.variant, gmode);
     long long plane_total = 0;
     for (int ci : g.members) {
       mcb::CaseDesc& d = cases[ci];

@@ -1544,20 +1544,18 @@ const void* phi_kernel_of(bool eq) {
             : reinterpret_cast<const void*>(k_phi<S, BX, BY>);
 }
 
+// The phi kernel of a variant and g form: the tile is the collide kernel's (stored g runs it
+// on the first update of a push run).
 template <class S>
-const void* phi_kernel(int variant, bool eq, dim3* block) {
-  switch (variant) {
-    case 0:
-    case kTmaVariant: *block = dim3(32, 8); return phi_kernel_of<S, 32, 8>(eq);
-    case 1: *block = dim3(16, 16); return phi_kernel_of<S, 16, 16>(eq);
-    // the pair variants' tiles are 64 x 4 cells (stored g runs this kernel on the first
-    // update of a push run)
-    case kPairVariant:
-    case kPairVariant + 1:
-    case 2: *block = dim3(64, 4); return phi_kernel_of<S, 64, 4>(eq);
-    case 3: *block = dim3(16, 8); return phi_kernel_of<S, 16, 8>(eq);
-    default: return nullptr;
-  }
+const void* phi_kernel(int variant, int gmode, dim3* block) {
+  const bool eq = gmode == kGEquil;
+  const Variant t = tile_of(variant, gmode);
+  *block = dim3(t.bx, t.by);
+  if (t.bx == 32 && t.by == 8) return phi_kernel_of<S, 32, 8>(eq);
+  if (t.bx == 16 && t.by == 16) return phi_kernel_of<S, 16, 16>(eq);
+  if (t.bx == 64 && t.by == 4) return phi_kernel_of<S, 64, 4>(eq);
+  if (t.bx == 16 && t.by == 8) return phi_kernel_of<S, 16, 8>(eq);
+  return nullptr;
 }
 
 template <class S, int GM>
@@ -1571,7 +1569,7 @@ const void* collide_kernel(int variant, dim3* block) {
     case kPairVariant + 1:
       // two cells per thread (the instance without the reference-mode shell; launches pick
       // by StepArgs::has_ref)
-      *block = dim3(kPairTX, kPairBY);
+      *block = dim3(PairShape<GM>::TX, PairShape<GM>::BY);
       return pair_kernel<S>(variant, false, GM, false);
     default: return nullptr;
   }
@@ -1679,7 +1677,7 @@ cudaError_t occupancy_of(int variant, int gmode, int qf, int ratio, int wide, in
                          int* collide_blocks) {
   if (!is_pair_variant(variant) && (qf == kQ27 || ratio || wide)) {
     dim3 bp;
-    const void* fp = phi_kernel<S>(0, gmode == kGEquil, &bp);
+    const void* fp = phi_kernel<S>(0, gmode, &bp);
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         phi_blocks, fp, static_cast<int>(bp.x * bp.y), 0);
     if (e != cudaSuccess) return e;
@@ -1689,7 +1687,7 @@ cudaError_t occupancy_of(int variant, int gmode, int qf, int ratio, int wide, in
   if (variant == kTmaVariant) {
     if (gmode != kGEquil) return cudaErrorInvalidValue;
     dim3 bp;
-    const void* fp = phi_kernel<S>(0, true, &bp);
+    const void* fp = phi_kernel<S>(0, gmode, &bp);
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         phi_blocks, fp, static_cast<int>(bp.x * bp.y), 0);
     if (e != cudaSuccess) return e;
@@ -1697,7 +1695,7 @@ cudaError_t occupancy_of(int variant, int gmode, int qf, int ratio, int wide, in
         collide_blocks, k_collide_tma<S>, kTmaBX * kTmaBY, TmaBox<typename S::FT>::kSmem);
   }
   dim3 bp, bc;
-  const void* fp = phi_kernel<S>(variant, gmode == kGEquil, &bp);
+  const void* fp = phi_kernel<S>(variant, gmode, &bp);
   const void* fc = collide_kernel_gm<S>(variant, gmode, &bc);
   if (!fp || !fc) return cudaErrorInvalidValue;
   cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -1733,7 +1731,8 @@ const void* collide_fn(int variant, int gmode, int qf, bool ratio, bool wide, bo
                        bool single, dim3* block, int* dyn) {
   *dyn = 0;
   if (is_pair_variant(variant)) {
-    *block = dim3(kPairTX, kPairBY);
+    const Variant tile = pair_tile(gmode);
+    *block = dim3(tile.bx / 2, tile.by);
     *dyn = pair_dyn_smem<S>(gmode);
     return pair_kernel<S>(variant, has_ref, gmode, single);
   }
@@ -1777,7 +1776,7 @@ cudaError_t residency_smem_of(int variant, int gmode, int qf, int ratio, int wid
   cudaError_t launch_phi_##suffix(int variant, int gmode, const StepArgs& a,               \
                                   cudaStream_t s) {                                        \
     dim3 block;                                                                            \
-    const void* fn = phi_kernel<S>(variant, gmode == kGEquil, &block);                     \
+    const void* fn = phi_kernel<S>(variant, gmode, &block);                                \
     return launch_on(fn, a.grid_phi, block, a, s);                                         \
   }                                                                                        \
   cudaError_t launch_collide_##suffix(int variant, int gmode, const StepArgs& a,           \

@@ -217,21 +217,33 @@ struct GPairIO<mcb::StB16> {
 namespace mcb {
 namespace {
 
-constexpr int kPairTX = 32;  // threads in x; a tile is 2 * kPairTX = 64 cells wide
+// Threads of a block in x and y: 32 x 4 (a tile of 64 x 4 cells), with relaxed g 16 x 8 (32 x 8
+// cells). The nearly square tile has fewer halo points (normals 340 for 256 cells against
+// 396, phi 432 against 544) but its warps cover two rows, so each f access touches as many
+// 32-byte sectors and half-used ones more often. Relaxed FP16 g, which stages g and the
+// previous phi with their halos, gains (128x128x256 243 us against 263), equilibrium g does
+// not (113.6 against 112.7).
+template <int GM>
+struct PairShape {
+  static constexpr int TX = GM == kGBgk ? 16 : 32, BY = GM == kGBgk ? 8 : 4;
+  static_assert(2 * TX == pair_tile(GM).bx && BY == pair_tile(GM).by, "the host's tile");
+};
 
 // Ring slot of a non-negative plane index in the 5-plane phi ring (unsigned: no sign fix-up).
 __device__ __forceinline__ unsigned slot5(int v) { return static_cast<unsigned>(v) % 5u; }
 
 // Dynamic shared memory of the relaxed-g pair kernel: two planes of staged g (18
-// populations x kPairBY rows x 34 words of two cells) and, for the 16-bit deviation form, a
-// ring of four planes of staged previous phi (kPairBY + 2 rows x 34 words).
+// populations x BY rows x TX + 2 words of two cells) and, for the 16-bit deviation form, a
+// ring of four planes of staged previous phi (BY + 2 rows x TX + 2 words).
 template <class S>
 __host__ __device__ constexpr int pair_gbuf_bytes() {
-  return 2 * (kQ - 1) * kPairBY * 2 * (kPairTX + 2) * static_cast<int>(sizeof(typename S::GT));
+  using P = PairShape<kGBgk>;
+  return 2 * (kQ - 1) * P::BY * 2 * (P::TX + 2) * static_cast<int>(sizeof(typename S::GT));
 }
 template <class S>
 __host__ __device__ constexpr int pair_bgk_smem() {
-  return pair_gbuf_bytes<S>() + (S::kDev ? 4 * (kPairBY + 2) * 2 * (kPairTX + 2) * 4 : 0);
+  using P = PairShape<kGBgk>;
+  return pair_gbuf_bytes<S>() + (S::kDev ? 4 * (P::BY + 2) * 2 * (P::TX + 2) * 4 : 0);
 }
 
 // kRef: some case of the launch is in reference mode (frozen shell); the shell handling is
@@ -244,7 +256,7 @@ __host__ __device__ constexpr int pair_bgk_smem() {
 // kGPop: stored at full relaxation; kGBgk: stored, pulled and relaxed with tau_g != 1). The
 // stored forms run periodic and wall modes only (no reference shell) and need 18 * cells
 // below 2^31 (checked on the host).
-template <class S, int BY, bool kRef, bool kL2, int GM, bool kOne>
+template <class S, bool kRef, bool kL2, int GM, bool kOne>
 __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Tile& t) {
   constexpr bool EQ = GM == kGEquil;
   constexpr bool BGK = GM == kGBgk;
@@ -258,7 +270,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
   using pk::mul;
   using pk::scale;
   using pk::sub;
-  constexpr int TX = kPairTX, BX = 2 * TX, NT = TX * BY;
+  constexpr int TX = PairShape<GM>::TX, BY = PairShape<GM>::BY, BX = 2 * TX, NT = TX * BY;
   constexpr int PX = BX + 4, PY = BY + 4, PP = PX * PY;  // phi plane, halo 2
   constexpr int PH = PX / 2, PP2 = PP / 2;              // the same in pairs of values
   constexpr int KP2 = (PP2 + NT - 1) / NT;              // phi pairs per thread per plane
@@ -622,18 +634,19 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
     if (z + 2 <= t.ze) normals(z + 2);
     if constexpr (kL2) {
       // Plane z + 2 (the source plane of the next update's cz = -1 populations): rows
-      // yt - 1 .. yt + BY of the tile's two 32-cell blocks, each a contiguous run of
-      // 19 x 32 values, in 128-byte lines spread over the block's threads.
+      // yt - 1 .. yt + BY of the tile's 32-cell blocks, each a contiguous run of 19 x 32
+      // values, in 128-byte lines spread over the block's threads.
       if (z + 2 < t.ze + 1) {
         const int zq = t.bc == kBcPeriodic ? wrap1(z + 2, nz) : min(z + 2, nz - 1);
         constexpr int kRunBytes = QF * 32 * static_cast<int>(sizeof(FT));
         constexpr int kLines = (kRunBytes + 127) / 128;
-        constexpr int kJobs = (BY + 2) * 2 * kLines;
+        constexpr int kXB = BX / 32;  // 32-cell blocks per row
+        constexpr int kJobs = (BY + 2) * kXB * kLines;
         const char* pl = reinterpret_cast<const char*>(fin + static_cast<long long>(zq) * PS);
         const int xb0 = t.xt >> 5;
         for (int j = tid; j < kJobs; j += NT) {
           const int line = j % kLines, rb = j / kLines;
-          const int row = rb >> 1, xb = xb0 + (rb & 1);
+          const int row = rb / kXB, xb = xb0 + rb % kXB;
           int yq = t.yt - 1 + row;
           yq = yq < 0 ? yq + ny : (yq >= ny ? yq - ny : yq);
           if (xb < t.fxb && yq >= 0 && yq < ny)
@@ -970,16 +983,17 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
   for (int q = max(t.ze - 2, t.zb - 1); q <= t.ze; ++q) flush(q);
 }
 
-template <class S, int BY, bool kRef, int kMinBlocks, bool kL2, int GM, bool kOne>
-__global__ void __launch_bounds__(kPairTX * BY, kMinBlocks)
+template <class S, bool kRef, int kMinBlocks, bool kL2, int GM, bool kOne>
+__global__ void __launch_bounds__(PairShape<GM>::TX * PairShape<GM>::BY, kMinBlocks)
     k_collide_pair(const __grid_constant__ StepArgs a) {
+  constexpr int BX = 2 * PairShape<GM>::TX, BY = PairShape<GM>::BY;
   grid_trigger();
   if constexpr (kOne) {
-    collide_pair_segment<S, BY, kRef, kL2, GM, true>(a, single_tile<2 * kPairTX, BY>(a));
+    collide_pair_segment<S, kRef, kL2, GM, true>(a, single_tile<BX, BY>(a));
     return;
   }
-  for_each_segment<2 * kPairTX, BY, true>(
-      a, [&](const Tile& t) { collide_pair_segment<S, BY, kRef, kL2, GM, false>(a, t); },
+  for_each_segment<BX, BY, true>(
+      a, [&](const Tile& t) { collide_pair_segment<S, kRef, kL2, GM, false>(a, t); },
       a.balanced != 0);
 }
 
@@ -996,19 +1010,19 @@ const void* pair_kernel_gm(int variant, bool with_ref) {
     constexpr int MB = (GM == kGBgk && !S::kDev) ? 2 : 3;
     return variant == kPairVariant
                ? reinterpret_cast<const void*>(
-                     k_collide_pair<S, kPairBY, false, MB, false, GM, kOne>)
+                     k_collide_pair<S, false, MB, false, GM, kOne>)
                : reinterpret_cast<const void*>(
-                     k_collide_pair<S, kPairBY, false, MB, true, GM, kOne>);
+                     k_collide_pair<S, false, MB, true, GM, kOne>);
   } else if (variant == kPairVariant) {
     return with_ref ? reinterpret_cast<const void*>(
-                          k_collide_pair<S, kPairBY, true, 3, false, GM, kOne>)
+                          k_collide_pair<S, true, 3, false, GM, kOne>)
                     : reinterpret_cast<const void*>(
-                          k_collide_pair<S, kPairBY, false, 3, false, GM, kOne>);
+                          k_collide_pair<S, false, 3, false, GM, kOne>);
   } else {
     return with_ref ? reinterpret_cast<const void*>(
-                          k_collide_pair<S, kPairBY, true, 3, true, GM, kOne>)
+                          k_collide_pair<S, true, 3, true, GM, kOne>)
                     : reinterpret_cast<const void*>(
-                          k_collide_pair<S, kPairBY, false, 3, true, GM, kOne>);
+                          k_collide_pair<S, false, 3, true, GM, kOne>);
   }
 }
 

@@ -148,8 +148,15 @@ constexpr Variant kVariants[kNumVariants] = {{32, 8}, {16, 16}, {64, 4}, {16, 8}
                                              {64, 4}, {64, 4}};
 constexpr int kTmaVariant = 4;
 constexpr int kPairVariant = 5;
-constexpr int kPairBY = 4;  // thread rows of the pair kernel's block
+// Tile of the pair kernel for a g form (relaxed g: 32 x 8 cells, see kernels_pair.cuh).
+constexpr Variant pair_tile(int gmode) {
+  return gmode == kGBgk ? Variant{32, 8} : Variant{64, 4};
+}
 constexpr bool is_pair_variant(int v) { return v == kPairVariant || v == kPairVariant + 1; }
+// Cell tile of a variant for a g form.
+constexpr Variant tile_of(int v, int gmode) {
+  return is_pair_variant(v) ? pair_tile(gmode) : kVariants[v];
+}
 constexpr int kErrTmaWait = 1;  // StepArgs::err: a TMA wait timed out
 constexpr int kDiagBlocks = 304;   // fixed grid: the reduction order never changes
 constexpr int kDiagThreads = 256;

@@ -203,6 +203,8 @@ int  mcb_write_info_file(const char* dir, const char* id, const char* velocity_s
                          double fy, double fz, int save_every, int nsteps, double mlups);
 
 /* The tile variant and z chunk setting the handle runs (after defaults and autotuning).
+ * variant 0 is the 32x8 tile, run with one cell per thread or (equilibrium g, D3Q19 f, an even
+ * nx, above 32^3 cells in all) with two, which gives the same fields bit for bit;
  * variant 4 is the TMA-staged 32x8 collide on the padded f layout; variant 5 takes two
  * neighbouring cells in x per thread (64x4 cells per block; D3Q19 f at density ratio 1 and
  * an even nx; with stored g also periodic or wall boundaries and 18 * cells < 2^31;

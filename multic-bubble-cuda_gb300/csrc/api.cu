@@ -132,6 +132,7 @@ struct Solver {
   int wide = 0;            // some case needs 64-bit f offsets
   bool padded = false;     // f in the padded layout of the TMA collide
   bool pair_ok = false;    // the two-cells-per-thread kernel can run these cases
+  bool pair_as0 = false;   // variant 0 runs its two-cells form (kPairAs0)
   bool wide_blocked = false;  // 64-bit f offsets on the blocked layout: the pair kernel only
   bool push = false;       // the collide kernel writes the next phi (all but the TMA kernel)
   CUtensorMap fmap[2];     // TMA descriptors of f[0], f[1] (padded only)
@@ -160,6 +161,7 @@ struct Solver {
   // splits it, is one group of every case with the handle's variant and z chunk request.
   struct Group {
     int variant = 0, zchunk_req = 0;
+    int kernel = 0;  // the variant's kernel: kPairAs0 for variant 0 where it applies
     std::vector<int> members;  // case indices, in launch order
     std::vector<int> zc_case;  // per member: > 0 fixed z chunk overriding the group's split
     int ntiles = 0, zchunk = 16, balanced = 1, phi_balanced = 0, planes = 0;
@@ -288,7 +290,8 @@ struct Solver {
   //   small cases (kBatchBalancedPlanes).
   // A member's own fixed chunk (zc_case > 0) overrides the group's unless it is balanced.
   int build_group(Group& g, int nsm) {
-    const mcb::Variant v = mcb::tile_of(g.variant, gmode);
+    g.kernel = g.variant == 0 && pair_as0 ? mcb::kPairAs0 : g.variant;
+    const mcb::Variant v = mcb::tile_of(g.kernel, gmode);
     long long plane_total = 0;
     for (int ci : g.members) {
       mcb::CaseDesc& d = cases[ci];
@@ -301,7 +304,7 @@ struct Solver {
     g.planes = static_cast<int>(plane_total);
     g.balanced = g.zchunk_req < 0;
     int occ_phi = 0, occ_col = 0;
-    MCB_CU(mcb::occupancy(storage, g.variant, gmode, qf, ratio, wide, &occ_phi, &occ_col));
+    MCB_CU(mcb::occupancy(storage, g.kernel, gmode, qf, ratio, wide, &occ_phi, &occ_col));
     if (occ_phi <= 0 || occ_col <= 0)
       return fail(MCB_ERR_CUDA, "no resident blocks for tile variant %d", g.variant);
     int zc = g.zchunk_req;
@@ -349,7 +352,8 @@ struct Solver {
     // (the y and z limits of a grid hold every lattice: at most 65535 cells per axis). 128 x
     // 128 x 256: 121.5 us against 123.0 at FP32, 110.3 against 112.7 at FP16; relaxed g stays
     // with the table (FP16 268 us against 264).
-    g.single = cases.size() == 1 && !g.balanced && mcb::is_pair_variant(g.variant) &&
+    g.single = cases.size() == 1 && !g.balanced &&
+               (g.kernel == mcb::kPairAs0 || mcb::is_pair_variant(g.variant)) &&
                gmode != mcb::kGBgk;
     return chain_of(g, nsm, occ_col);
   }
@@ -372,7 +376,7 @@ struct Solver {
       return MCB_OK;
     const int per_sm = (g.grid_collide + nsm - 1) / nsm;
     if (per_sm < occ_col)
-      MCB_CU(mcb::residency_smem(storage, g.variant, gmode, qf, ratio, wide, g.has_ref, g.single,
+      MCB_CU(mcb::residency_smem(storage, g.kernel, gmode, qf, ratio, wide, g.has_ref, g.single,
                                  per_sm, &g.smem));
     g.chain = per_sm >= occ_col || g.smem > 0;
     return MCB_OK;
@@ -504,6 +508,12 @@ struct Solver {
         pair_ok = pair_ok && d.bc != mcb::kBcRef && 18LL * d.ncell < (1LL << 31);
     }
     if (mcb::is_pair_variant(variant) && !pair_ok) variant = 0;
+    // Tile variant 0 with equilibrium g runs two cells per thread (same fields, bit for bit)
+    // above 32^3 cells: 64 FP16 cases of 32..96 cells 676 us per update against 810, 96^3 FP16
+    // 26.6 against 32.5 and FP32 30.2 against 33.1, 160^3 FP16 106 against 130, 48^3 FP32 8.6
+    // against 9.2. At 32^3 both take 5.7 us, at 24^3 one cell per thread is faster (5.5
+    // against 5.6): too few warps for longer ones.
+    pair_as0 = pair_ok && gmode == mcb::kGEquil && !wide && cells_total > (1LL << 15);
     // Default tile: the pair kernel where it applies, else 32x8. Measured on GB300, collide
     // kernel of the 128x128x256 walls-and-gravity workload (FP32 / FP16 / BF16 storage):
     //   - equilibrium g: 133 us against 137 at FP32, 120 against 138 at FP16;
@@ -806,14 +816,14 @@ struct Solver {
   int launch_phi_stage(bool with_macros) {
     if (skips_phi()) return MCB_OK;
     for (const auto& gr : groups)
-      MCB_CU(mcb::launch_phi(storage, gr.variant, gmode, args(gr, with_macros), stream));
+      MCB_CU(mcb::launch_phi(storage, gr.kernel, gmode, args(gr, with_macros), stream));
     return MCB_OK;
   }
 
   // The collide kernels of the groups.
   int launch_collide_stage(bool with_macros) {
     for (const auto& gr : groups)
-      MCB_CU(mcb::launch_collide(storage, gr.variant, gmode, args(gr, with_macros),
+      MCB_CU(mcb::launch_collide(storage, gr.kernel, gmode, args(gr, with_macros),
                                  padded ? &fmap[parity] : nullptr, stream));
     return MCB_OK;
   }

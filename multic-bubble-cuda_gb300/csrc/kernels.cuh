@@ -1569,7 +1569,7 @@ const void* collide_kernel(int variant, dim3* block) {
     case kPairVariant + 1:
       // two cells per thread (the instance without the reference-mode shell; launches pick
       // by StepArgs::has_ref)
-      *block = dim3(PairShape<GM>::TX, PairShape<GM>::BY);
+      *block = dim3(PairShape<GM, false>::TX, PairShape<GM, false>::BY);
       return pair_kernel<S>(variant, false, GM, false);
     default: return nullptr;
   }
@@ -1675,6 +1675,16 @@ inline cudaError_t opt_in_smem(const void* fn, int* largest = nullptr) {
 template <class S>
 cudaError_t occupancy_of(int variant, int gmode, int qf, int ratio, int wide, int* phi_blocks,
                          int* collide_blocks) {
+  if (variant == kPairAs0) {
+    dim3 bp;
+    const void* fp = phi_kernel<S>(variant, gmode, &bp);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        phi_blocks, fp, static_cast<int>(bp.x * bp.y), 0);
+    if (e != cudaSuccess) return e;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        collide_blocks, pair_kernel_rc<S>(false, false), kVariants[0].bx / 2 * kVariants[0].by,
+        0);
+  }
   if (!is_pair_variant(variant) && (qf == kQ27 || ratio || wide)) {
     dim3 bp;
     const void* fp = phi_kernel<S>(0, gmode, &bp);
@@ -1730,6 +1740,10 @@ template <class S>
 const void* collide_fn(int variant, int gmode, int qf, bool ratio, bool wide, bool has_ref,
                        bool single, dim3* block, int* dyn) {
   *dyn = 0;
+  if (variant == kPairAs0) {
+    *block = dim3(kVariants[0].bx / 2, kVariants[0].by);
+    return pair_kernel_rc<S>(has_ref, single);
+  }
   if (is_pair_variant(variant)) {
     const Variant tile = pair_tile(gmode);
     *block = dim3(tile.bx / 2, tile.by);

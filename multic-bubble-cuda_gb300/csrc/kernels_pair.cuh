@@ -223,10 +223,10 @@ namespace {
 // 32-byte sectors and half-used ones more often. Relaxed FP16 g, which stages g and the
 // previous phi with their halos, gains (128x128x256 243 us against 263), equilibrium g does
 // not (113.6 against 112.7).
-template <int GM>
+template <int GM, bool RC>
 struct PairShape {
-  static constexpr int TX = GM == kGBgk ? 16 : 32, BY = GM == kGBgk ? 8 : 4;
-  static_assert(2 * TX == pair_tile(GM).bx && BY == pair_tile(GM).by, "the host's tile");
+  static constexpr int TX = RC || GM == kGBgk ? 16 : 32, BY = RC || GM == kGBgk ? 8 : 4;
+  static_assert(RC || (2 * TX == pair_tile(GM).bx && BY == pair_tile(GM).by), "the host's tile");
 };
 
 // Ring slot of a non-negative plane index in the 5-plane phi ring (unsigned: no sign fix-up).
@@ -237,12 +237,12 @@ __device__ __forceinline__ unsigned slot5(int v) { return static_cast<unsigned>(
 // ring of four planes of staged previous phi (BY + 2 rows x TX + 2 words).
 template <class S>
 __host__ __device__ constexpr int pair_gbuf_bytes() {
-  using P = PairShape<kGBgk>;
+  using P = PairShape<kGBgk, false>;
   return 2 * (kQ - 1) * P::BY * 2 * (P::TX + 2) * static_cast<int>(sizeof(typename S::GT));
 }
 template <class S>
 __host__ __device__ constexpr int pair_bgk_smem() {
-  using P = PairShape<kGBgk>;
+  using P = PairShape<kGBgk, false>;
   return pair_gbuf_bytes<S>() + (S::kDev ? 4 * (P::BY + 2) * 2 * (P::TX + 2) * 4 : 0);
 }
 
@@ -252,11 +252,16 @@ __host__ __device__ constexpr int pair_bgk_smem() {
 // kOne: the launch holds one case in fixed chunks, described by the kernel's parameters: the
 // per-plane bases and bounds then come from uniform registers and constants (508 warp
 // instructions per 32 cells against 532 at FP16, 110.3 us against 112.7 on 128x128x256).
+// RC: rounds every step as the one-cell kernel (k_collide, as the compiler fuses its
+// expressions) does, on that kernel's 32 x 8-cell tile, so that tile variant 0 gives the same
+// fields, bit for bit, from either: the curvature neighbour by neighbour, the force as (sigma
+// kappa n) |grad phi|, and the fused multiply-adds of u.F, u^2, Pi, f* and J in the order
+// marked RC below (equilibrium g; measured where the host picks it).
 // GM: how g crosses the update (kGEquil: pushed equilibrium populations, nothing stored;
 // kGPop: stored at full relaxation; kGBgk: stored, pulled and relaxed with tau_g != 1). The
 // stored forms run periodic and wall modes only (no reference shell) and need 18 * cells
 // below 2^31 (checked on the host).
-template <class S, bool kRef, bool kL2, int GM, bool kOne>
+template <class S, bool kRef, bool kL2, int GM, bool kOne, bool RC>
 __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Tile& t) {
   constexpr bool EQ = GM == kGEquil;
   constexpr bool BGK = GM == kGBgk;
@@ -270,7 +275,8 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
   using pk::mul;
   using pk::scale;
   using pk::sub;
-  constexpr int TX = PairShape<GM>::TX, BY = PairShape<GM>::BY, BX = 2 * TX, NT = TX * BY;
+  using Shape = PairShape<GM, RC>;
+  constexpr int TX = Shape::TX, BY = Shape::BY, BX = 2 * TX, NT = TX * BY;
   constexpr int PX = BX + 4, PY = BY + 4, PP = PX * PY;  // phi plane, halo 2
   constexpr int PH = PX / 2, PP2 = PP / 2;              // the same in pairs of values
   constexpr int KP2 = (PP2 + NT - 1) / NT;              // phi pairs per thread per plane
@@ -675,27 +681,53 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
     };
     const float2 ncx = nrm2(n0, 0, 0), ncy = nrm2(n0, 1, 0), ncz = nrm2(n0, 2, 0);
     const float2 ncw = nrm2(n0, 3, 0);
-    // Per opposite pair (l, l + 1): W_l c_l . (n(x + c_l) - n(x - c_l)).
     float2 kap = dup(0.f);
-    static_for<0, (kQ - 1) / 2>([&](auto KC) {
-      constexpr int L = 2 * decltype(KC)::value + 1;
-      constexpr float w3 = 3.0f * wf(L);
-      const float(*pp)[HP] = nbr_of<cz(L)>(nm, n0, np);   // x + c_l
-      const float(*pq)[HP] = nbr_of<-cz(L)>(nm, n0, np);  // x - c_l
-      constexpr int o = cy(L) * HX + cx(L);
-      const float2 cp = pk::cdot<cx(L), cy(L), cz(L)>(
-          cx(L) ? nrm2(pp, 0, o) : dup(0.f), cy(L) ? nrm2(pp, 1, o) : dup(0.f),
-          cz(L) ? nrm2(pp, 2, o) : dup(0.f));
-      const float2 cm = pk::cdot<cx(L), cy(L), cz(L)>(
-          cx(L) ? nrm2(pq, 0, -o) : dup(0.f), cy(L) ? nrm2(pq, 1, -o) : dup(0.f),
-          cz(L) ? nrm2(pq, 2, -o) : dup(0.f));
-      if constexpr (L == 1) kap = mul(dup(-w3), sub(cp, cm));
-      else kap = fma(dup(-w3), sub(cp, cm), kap);
-    });
+    if constexpr (RC) {
+      // neighbour by neighbour
+      static_for<1, kQ>([&](auto LC) {
+        constexpr int L = decltype(LC)::value;
+        constexpr float w3 = 3.0f * wf(L);
+        const float(*pl)[HP] = nbr_of<cz(L)>(nm, n0, np);
+        constexpr int o = cy(L) * HX + cx(L);
+        // c.n up to the sign of its first term, which the weight takes
+        constexpr int s1 = cx(L) != 0 ? cx(L) : (cy(L) != 0 ? cy(L) : cz(L));
+        const float2 cn = pk::cdot<cx(L) * s1, cy(L) * s1, cz(L) * s1>(
+            cx(L) ? nrm2(pl, 0, o) : dup(0.f), cy(L) ? nrm2(pl, 1, o) : dup(0.f),
+            cz(L) ? nrm2(pl, 2, o) : dup(0.f));
+        if constexpr (L == 1) kap = mul(dup(-w3 * s1), cn);
+        else kap = fma(dup(-w3 * s1), cn, kap);
+      });
+    } else {
+      // Per opposite pair (l, l + 1): W_l c_l . (n(x + c_l) - n(x - c_l)).
+      static_for<0, (kQ - 1) / 2>([&](auto KC) {
+        constexpr int L = 2 * decltype(KC)::value + 1;
+        constexpr float w3 = 3.0f * wf(L);
+        const float(*pp)[HP] = nbr_of<cz(L)>(nm, n0, np);   // x + c_l
+        const float(*pq)[HP] = nbr_of<-cz(L)>(nm, n0, np);  // x - c_l
+        constexpr int o = cy(L) * HX + cx(L);
+        const float2 cp = pk::cdot<cx(L), cy(L), cz(L)>(
+            cx(L) ? nrm2(pp, 0, o) : dup(0.f), cy(L) ? nrm2(pp, 1, o) : dup(0.f),
+            cz(L) ? nrm2(pp, 2, o) : dup(0.f));
+        const float2 cm = pk::cdot<cx(L), cy(L), cz(L)>(
+            cx(L) ? nrm2(pq, 0, -o) : dup(0.f), cy(L) ? nrm2(pq, 1, -o) : dup(0.f),
+            cz(L) ? nrm2(pq, 2, -o) : dup(0.f));
+        if constexpr (L == 1) kap = mul(dup(-w3), sub(cp, cm));
+        else kap = fma(dup(-w3), sub(cp, cm), kap);
+      });
+    }
     const float2 phi = *reinterpret_cast<const float2*>(&sphi[slot5(z + 5)][(ty + 2) * PX + 2 * tx + 2]);
     const float2 mult = scale(kap, sigma);
-    const float2 mw = mul(mult, ncw);
-    float2 Fx = mul(mw, ncx), Fy = mul(mw, ncy), Fz = mul(mw, ncz);
+    float2 Fx, Fy, Fz;
+    if constexpr (RC) {
+      Fx = mul(mul(mult, ncx), ncw);
+      Fy = mul(mul(mult, ncy), ncw);
+      Fz = mul(mul(mult, ncz), ncw);
+    } else {
+      const float2 mw = mul(mult, ncw);
+      Fx = mul(mw, ncx);
+      Fy = mul(mw, ncy);
+      Fz = mul(mw, ncz);
+    }
     if (gravity != 0.f) Fz = fma(dup(gravity), sub(phi, dup(phi_mean)), Fz);
 
     // Moments (momentiCalc, src/lbm.cu:133-225), from opposite-pair sums; deviation storage
@@ -733,19 +765,40 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
     const float2 ux = mul(fma(dup(0.5f), Fx, jx), inv_rho);
     const float2 uy = mul(fma(dup(0.5f), Fy, jy), inv_rho);
     const float2 uz = mul(fma(dup(0.5f), Fz, jz), inv_rho);
-    const float2 uF = fma(uz, Fz, fma(uy, Fy, mul(ux, Fx)));
+    const float2 uF = RC ? fma(uz, Fz, fma(ux, Fx, mul(uy, Fy)))
+                         : fma(uz, Fz, fma(uy, Fy, mul(ux, Fx)));
     const float2 nh = scale(uF, -1.5f);  // -h
     const float2 nrho = scale(rho, -1.0f);
-    const float2 uxx = mul(ux, ux), uyy = mul(uy, uy), uzz = mul(uz, uz);
-    const float2 uxy = mul(ux, uy), uxz = mul(ux, uz), uyz = mul(uy, uz);
+    float2 pxx, pyy, pzz, pxy, pxz, pyz, u2;
     // p_ab = s_ab - rho (d_ab / 3 + u_a u_b) + (u_a F_b + u_b F_a) / 2 - h u_a u_b
-    const float2 pxx = fma(nh, uxx, fma(ux, Fx, fma(nrho, add(dup(1.0f / 3.0f), uxx), sxx)));
-    const float2 pyy = fma(nh, uyy, fma(uy, Fy, fma(nrho, add(dup(1.0f / 3.0f), uyy), syy)));
-    const float2 pzz = fma(nh, uzz, fma(uz, Fz, fma(nrho, add(dup(1.0f / 3.0f), uzz), szz)));
-    const float2 pxy = fma(nh, uxy, fma(dup(0.5f), fma(ux, Fy, mul(uy, Fx)), fma(nrho, uxy, sxy)));
-    const float2 pxz = fma(nh, uxz, fma(dup(0.5f), fma(ux, Fz, mul(uz, Fx)), fma(nrho, uxz, sxz)));
-    const float2 pyz = fma(nh, uyz, fma(dup(0.5f), fma(uy, Fz, mul(uz, Fy)), fma(nrho, uyz, syz)));
-    const float2 u2 = add(add(uxx, uyy), uzz);
+    if constexpr (RC) {
+      const float2 hx = mul(nh, ux), hy = mul(nh, uy), hz = mul(nh, uz);
+      const float2 rx = mul(nrho, ux), ry = mul(nrho, uy);
+      auto diag = [&](float2 u, float2 F, float2 h, float2 sv) {
+        return fma(h, u, fma(u, F, fma(nrho, add(dup(1.0f / 3.0f), mul(u, u)), sv)));
+      };
+      auto off = [&](float2 ua, float2 Fa, float2 ub, float2 Fb, float2 ra, float2 ha,
+                     float2 sv) {
+        return fma(ha, ub, fma(dup(0.5f), fma(ua, Fb, mul(ub, Fa)), fma(ra, ub, sv)));
+      };
+      pxx = diag(ux, Fx, hx, sxx);
+      pyy = diag(uy, Fy, hy, syy);
+      pzz = diag(uz, Fz, hz, szz);
+      pxy = off(ux, Fx, uy, Fy, rx, hx, sxy);
+      pxz = off(ux, Fx, uz, Fz, rx, hx, sxz);
+      pyz = off(uy, Fy, uz, Fz, ry, hy, syz);
+      u2 = fma(uz, uz, fma(ux, ux, mul(uy, uy)));
+    } else {
+      const float2 uxx = mul(ux, ux), uyy = mul(uy, uy), uzz = mul(uz, uz);
+      const float2 uxy = mul(ux, uy), uxz = mul(ux, uz), uyz = mul(uy, uz);
+      pxx = fma(nh, uxx, fma(ux, Fx, fma(nrho, add(dup(1.0f / 3.0f), uxx), sxx)));
+      pyy = fma(nh, uyy, fma(uy, Fy, fma(nrho, add(dup(1.0f / 3.0f), uyy), syy)));
+      pzz = fma(nh, uzz, fma(uz, Fz, fma(nrho, add(dup(1.0f / 3.0f), uzz), szz)));
+      pxy = fma(nh, uxy, fma(dup(0.5f), fma(ux, Fy, mul(uy, Fx)), fma(nrho, uxy, sxy)));
+      pxz = fma(nh, uxz, fma(dup(0.5f), fma(ux, Fz, mul(uz, Fx)), fma(nrho, uxz, sxz)));
+      pyz = fma(nh, uyz, fma(dup(0.5f), fma(uy, Fz, mul(uz, Fy)), fma(nrho, uyz, syz)));
+      u2 = add(add(uxx, uyy), uzz);
+    }
     const float2 tr3 = scale(add(add(pxx, pyy), pzz), 1.0f / 3.0f);
 
     // Regularized collision with He forcing (collisionFluid, src/lbm.cu:233-288):
@@ -833,7 +886,11 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
       }
       IO::st2(fo_base + L * 32, v);
     };
-    {
+    if constexpr (RC) {
+      float2 v = fma(base, R, scale(mul(om, tr3), -1.0f));
+      if constexpr (kDevF) v = add(v, dup(fshift));
+      put(0, scale(v, wf(0)));
+    } else {
       const float2 v = scale(fma(base, R, fma(scale(om, -1.0f), tr3, dup(fshift))), wf(0));
       put(0, v);
     }
@@ -851,10 +908,17 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
       if constexpr (cx(L) * cz(L) != 0) qp = fma(dup(2.0f * cx(L) * cz(L)), pxz, qp);
       if constexpr (cy(L) * cz(L) != 0) qp = fma(dup(2.0f * cy(L) * cz(L)), pyz, qp);
       const float2 q = fma(om, qp, dup(fshift));
-      const float2 e0 = fma(scale(cu, 4.5f), cu, base), e1 = scale(cu, 3.0f);
-      const float2 rf = scale(cF, 1.5f);
-      put(L, scale(fma(add(e0, e1), add(R, rf), q), W));
-      put(O, scale(fma(sub(e0, e1), sub(R, rf), q), W));
+      const float2 e0 = fma(scale(cu, 4.5f), cu, base);
+      if constexpr (RC) {
+        const float2 ea = fma(dup(3.0f), cu, e0), eb = fma(dup(-3.0f), cu, e0);
+        const float2 ra = fma(dup(1.5f), cF, R), rb = fma(dup(-1.5f), cF, R);
+        put(L, scale(fma(ea, ra, q), W));
+        put(O, scale(fma(eb, rb, q), W));
+      } else {
+        const float2 e1 = scale(cu, 3.0f), rf = scale(cF, 1.5f);
+        put(L, scale(fma(add(e0, e1), add(R, rf), q), W));
+        put(O, scale(fma(sub(e0, e1), sub(R, rf), q), W));
+      }
     });
     if constexpr (!EQ) {
       // Stored g, after the f collision (fewer values live at once): W_l (phi +- dg),
@@ -886,9 +950,10 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
       // equilibrium W_l (phi + c_l.J), J = 3 phi u + sharp_c phi (1 - phi) n, pushed as exact
       // Q2.30 integers into the next phi (streamingCalc + phiCalc).
       constexpr float kj = 1073741824.0f / 36.0f;
-      const float2 Jx = scale(fma(phi3, ux, mul(A, ncx)), kj);
-      const float2 Jy = scale(fma(phi3, uy, mul(A, ncy)), kj);
-      const float2 Jz = scale(fma(phi3, uz, mul(A, ncz)), kj);
+      auto flux = [&](float2 u, float2 n) {
+        return scale(RC ? fma(A, n, mul(phi3, u)) : fma(phi3, u, mul(A, n)), kj);
+      };
+      const float2 Jx = flux(ux, ncx), Jy = flux(uy, ncy), Jz = flux(uz, ncz);
       // shell lanes push their phi with no flux
       JQ j0{__float2int_rn(Jx.x), __float2int_rn(Jy.x), __float2int_rn(Jz.x)};
       JQ j1{__float2int_rn(Jx.y), __float2int_rn(Jy.y), __float2int_rn(Jz.y)};
@@ -983,17 +1048,17 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
   for (int q = max(t.ze - 2, t.zb - 1); q <= t.ze; ++q) flush(q);
 }
 
-template <class S, bool kRef, int kMinBlocks, bool kL2, int GM, bool kOne>
-__global__ void __launch_bounds__(PairShape<GM>::TX * PairShape<GM>::BY, kMinBlocks)
+template <class S, bool kRef, int kMinBlocks, bool kL2, int GM, bool kOne, bool RC = false>
+__global__ void __launch_bounds__(PairShape<GM, RC>::TX * PairShape<GM, RC>::BY, kMinBlocks)
     k_collide_pair(const __grid_constant__ StepArgs a) {
-  constexpr int BX = 2 * PairShape<GM>::TX, BY = PairShape<GM>::BY;
+  constexpr int BX = 2 * PairShape<GM, RC>::TX, BY = PairShape<GM, RC>::BY;
   grid_trigger();
   if constexpr (kOne) {
-    collide_pair_segment<S, kRef, kL2, GM, true>(a, single_tile<BX, BY>(a));
+    collide_pair_segment<S, kRef, kL2, GM, true, RC>(a, single_tile<BX, BY>(a));
     return;
   }
   for_each_segment<BX, BY, true>(
-      a, [&](const Tile& t) { collide_pair_segment<S, kRef, kL2, GM, false>(a, t); },
+      a, [&](const Tile& t) { collide_pair_segment<S, kRef, kL2, GM, false, RC>(a, t); },
       a.balanced != 0);
 }
 
@@ -1024,6 +1089,20 @@ const void* pair_kernel_gm(int variant, bool with_ref) {
                     : reinterpret_cast<const void*>(
                           k_collide_pair<S, false, 3, true, GM, kOne>);
   }
+}
+
+// The pair kernel that rounds as the one-cell 32x8 kernel does (equilibrium g).
+template <class S>
+const void* pair_kernel_rc(bool with_ref, bool single) {
+  if (single)
+    return with_ref ? reinterpret_cast<const void*>(
+                          k_collide_pair<S, true, 3, false, kGEquil, true, true>)
+                    : reinterpret_cast<const void*>(
+                          k_collide_pair<S, false, 3, false, kGEquil, true, true>);
+  return with_ref ? reinterpret_cast<const void*>(
+                        k_collide_pair<S, true, 3, false, kGEquil, false, true>)
+                  : reinterpret_cast<const void*>(
+                        k_collide_pair<S, false, 3, false, kGEquil, false, true>);
 }
 
 // Dynamic shared memory of a pair-kernel launch.

@@ -152,9 +152,14 @@ constexpr int kPairVariant = 5;
 constexpr Variant pair_tile(int gmode) {
   return gmode == kGBgk ? Variant{32, 8} : Variant{64, 4};
 }
+// The kernel that runs tile variant 0 where two cells per thread apply (solver-internal, not
+// a variant that callers name): the pair kernel on 32 x 8 cells with the one-cell kernel's
+// rounding, so that variant 0 gives the same fields bit for bit whichever of the two runs.
+constexpr int kPairAs0 = kNumVariants;
 constexpr bool is_pair_variant(int v) { return v == kPairVariant || v == kPairVariant + 1; }
 // Cell tile of a variant for a g form.
 constexpr Variant tile_of(int v, int gmode) {
+  if (v == kPairAs0) return kVariants[0];
   return is_pair_variant(v) ? pair_tile(gmode) : kVariants[v];
 }
 constexpr int kErrTmaWait = 1;  // StepArgs::err: a TMA wait timed out

@@ -53,3 +53,17 @@ def test_small_batch_runs_balanced_and_keeps_the_fields():
             out.append([b.get(i, "phi") for i in range(len(cfgs))])
     for a, c in zip(*out):
         assert np.array_equal(a, c)
+
+
+# above and below the size where tile variant 0 takes two cells per thread; ragged in x and y,
+# one tile wide, wall and shell planes in the first and the last chunk
+@pytest.mark.parametrize("dims", [(34, 33, 30), (96, 30, 12), (30, 50, 40), (32, 32, 32)])
+@pytest.mark.parametrize("storage", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("bc", [mcb.BC_PERIODIC, mcb.BC_WALLS_Z, mcb.BC_REF])
+def test_tile_0_with_two_cells_per_thread_rounds_as_the_one_cell_tiles(dims, storage, bc):
+    kw = dict(nx=dims[0], ny=dims[1], nz=dims[2], bc=bc, storage=storage, tau=0.65, sigma=0.3,
+              sharp_c=0.0, gravity=0.0 if bc == mcb.BC_REF else 1e-3)
+    ref = _run(mcb.default_config(variant=3, **kw))
+    got = _run(mcb.default_config(variant=0, **kw))
+    assert got[0][0] == 0 and ref[0][0] == 3
+    assert np.array_equal(ref[1], got[1]) and np.array_equal(ref[2], got[2])

@@ -681,7 +681,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
     else if (walls) z = z < 0 ? -1 - z : (z >= nz ? 2 * nz - 1 - z : z);  // mirror
     return clampi(z, 0, nz - 1);
   };
-  int pre[KPF];
+  int pre[KPF] = {};
   auto issue = [&](int zpl) {
     const int* base = pcur + static_cast<long long>(zmap(zpl)) * nxy;
 #pragma unroll
@@ -840,7 +840,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
   constexpr bool kPRing = BGK && S::kDev && !kTma && kSmemNoRing + 16 * HP <= 48 * 1024;
   constexpr int KPR = kPRing ? (HP + NT - 1) / NT : 1;
   __shared__ int sprev[kPRing ? 4 : 1][kPRing ? HP : 1];
-  int proff[KPR], ppre[KPR];
+  int proff[KPR] = {}, ppre[KPR] = {};
   if constexpr (kPRing) {
 #pragma unroll
     for (int k = 0; k < KPR; ++k) {
@@ -934,15 +934,40 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
   // z-1 .. z+1.
   if constexpr (!kTma) grid_wait();
   // Prologue: phi planes zb-2 .. zb+2, normals zb-1 .. zb+1.
-  for (int zpl = t.zb - 2; zpl <= t.zb + 2; ++zpl) {
-    issue(zpl);
-    commit(zpl);
+  // The loads of all five phi planes (and of the three previous-phi planes) are in flight
+  // together: one trip to memory instead of five in a row.
+  {
+    int first[5][KPF], prev_first[3][KPR];
+#pragma unroll
+    for (int p = 0; p < 5; ++p) {
+      issue(t.zb - 2 + p);
+#pragma unroll
+      for (int k = 0; k < KPF; ++k) first[p][k] = pre[k];
+    }
+    if constexpr (kPRing) {
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        prev_issue(t.zb - 1 + p);
+#pragma unroll
+        for (int k = 0; k < KPR; ++k) prev_first[p][k] = ppre[k];
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < 5; ++p) {
+#pragma unroll
+      for (int k = 0; k < KPF; ++k) pre[k] = first[p][k];
+      commit(t.zb - 2 + p);
+    }
+    if constexpr (kPRing) {
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+#pragma unroll
+        for (int k = 0; k < KPR; ++k) ppre[k] = prev_first[p][k];
+        prev_commit(t.zb - 1 + p);
+      }
+    }
   }
   issue(t.zb + 3);
-  for (int q = t.zb - 1; q <= t.zb + 1; ++q) {
-    prev_issue(q);
-    prev_commit(q);
-  }
   prev_issue(t.zb + 2);
   __syncthreads();
   for (int zpl = t.zb - 1; zpl <= t.zb + 1; ++zpl) normals(zpl);

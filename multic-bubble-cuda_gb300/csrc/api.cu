@@ -514,18 +514,18 @@ struct Solver {
     // against 9.2. At 32^3 both take 5.7 us, at 24^3 one cell per thread is faster (5.5
     // against 5.6): too few warps for longer ones.
     pair_as0 = pair_ok && gmode == mcb::kGEquil && !wide && cells_total > (1LL << 15);
-    // Default tile: the pair kernel where it applies, else 32x8. Measured on GB300, collide
-    // kernel of the 128x128x256 walls-and-gravity workload (FP32 / FP16 / BF16 storage):
-    //   - equilibrium g: 133 us against 137 at FP32, 120 against 138 at FP16;
-    //   - g stored at full relaxation: 163 / 147 / 156 us against 174 / 171 / 198;
-    //   - relaxed g (tau_g 0.8): 16-bit storage with the L2 prefetch variant, 275 / 303 us
-    //     against 298 / 313; at FP32 the one-cell tile stays (233 us against 286).
-    // Where nx leaves the pair kernel's 64-cell-wide tiles emptier than the one-cell
-    // kernel's 32-wide ones, the one-cell tile stays: 96^3, equilibrium g, 35.6 us against
-    // 41.0 (FP32); 80^3 27.9 against 31.9. 200x200x100 (tiles 78 % full, against 89 %)
-    // still runs the pair kernel faster, 157 us against 175. Stored g takes the pair kernel
-    // from 64^3 (there 16.6 us against 17.8 for the populations at FP32, 25.1 against 26.0
-    // relaxed at FP16); 32^3 and 96^3 run faster one cell per thread.
+    // Default tile: the pair kernel where it applies, else variant 0. Measured on GB300, us
+    // per update of the 128x128x256 walls-and-gravity workload (FP32 / FP16 / BF16 storage),
+    // pair kernel against one cell per thread:
+    //   - equilibrium g: 120 against 134 at FP32, 109 against 135 at FP16;
+    //   - g stored at full relaxation: 160 against 174 at FP32;
+    //   - relaxed g (tau_g 0.8): 16-bit storage with the L2 prefetch variant, 241 / 269 us
+    //     against 287 / 307; at FP32 the one-cell tile stays (228 us against 256).
+    // Where nx leaves the pair kernel's 64-cell-wide tiles emptier than 32-wide ones, variant
+    // 0 stays: 96^3, equilibrium g, 30.2 us against 37.8 (FP32), 26.6 against 35.7 (FP16); 80^3
+    // 23.0 against 29.0. 200x200x100 (tiles 78 % full, against 89 %) runs the pair kernel.
+    // Stored g takes the pair kernel from 64^3 (there 24.8 us against 25.9 relaxed at FP16,
+    // at 32^3 10.6 against 8.2); where the line lies between them, fields would change with it.
     auto x_fill = [&](int w) {  // share of the tiles' thread columns that hold cells
       double c = 0, t = 0;
       for (auto& d : cases) {

@@ -206,7 +206,8 @@ int  mcb_write_info_file(const char* dir, const char* id, const char* velocity_s
  * variant 0 is the 32x8 tile, run with one cell per thread or (equilibrium g, D3Q19 f, an even
  * nx, above 32^3 cells in all) with two, which gives the same fields bit for bit;
  * variant 4 is the TMA-staged 32x8 collide on the padded f layout; variant 5 takes two
- * neighbouring cells in x per thread (64x4 cells per block; D3Q19 f at density ratio 1 and
+ * neighbouring cells in x per thread (64x4 cells per block, 32x8 with relaxed g; D3Q19 f at
+ * density ratio 1 and
  * an even nx; with stored g also periodic or wall boundaries and 18 * cells < 2^31;
  * elsewhere a request for it runs variant 0), and variant 6 is variant 5 with an L2
  * prefetch of the f rows of the plane after next. Defaults: variant 5 where it applies

@@ -67,8 +67,8 @@ struct StF32 {
   using GT = int;
   static constexpr bool kDev = false;   // g decode needs the source cell's phi
   static constexpr bool kFDev = false;  // f stored as f_l - W_l
-  static __device__ __forceinline__ FT fload(const FT* p) { return __ldg(p); }
-  static __device__ __forceinline__ GT gload(const GT* p) { return __ldg(p); }
+  static __device__ __forceinline__ FT fload(const FT* p) { return *p; }
+  static __device__ __forceinline__ GT gload(const GT* p) { return *p; }
   template <int L> static __device__ __forceinline__ float f_raw(FT v) { return v; }
   template <int L> static __device__ __forceinline__ FT f_put(float f) { return f; }
   template <int L> static __device__ __forceinline__ int g_dec(GT v, int) { return v; }
@@ -119,8 +119,8 @@ struct St16 {
   using GT = typename O::T;
   static constexpr bool kDev = true;
   static constexpr bool kFDev = true;
-  static __device__ __forceinline__ FT fload(const FT* p) { return __ldg(p); }
-  static __device__ __forceinline__ GT gload(const GT* p) { return __ldg(p); }
+  static __device__ __forceinline__ FT fload(const FT* p) { return *p; }
+  static __device__ __forceinline__ GT gload(const GT* p) { return *p; }
   template <int L> static __device__ __forceinline__ float f_raw(FT v) { return O::tof(v); }
   template <int L> static __device__ __forceinline__ FT f_put(float dev) {
     return O::fromf(dev);
@@ -185,6 +185,9 @@ __device__ __forceinline__ void l2_prefetch(const void* p) {
 // be launched as soon as every block of this one has started, and waits for the previous
 // kernel (complete, its writes visible) before its first access to the lattice. The launch
 // and the set-up of the offsets then run under the previous update's last blocks.
+// So a block may be alive while the kernel before it still writes phi, f and g. The read-only
+// path (__ldg, const __restrict__) is for data that nothing writes during a kernel's life:
+// here the case table alone. Phi, f and g go by plain loads, which stay behind the wait.
 __device__ __forceinline__ void grid_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -334,9 +337,9 @@ __device__ __forceinline__ void phi_segment(const StepArgs& a, const Tile& t) {
   const int y = t.yt + static_cast<int>(threadIdx.y);
   if (x >= nx || y >= ny) return;
   const long long n = t.ncell;
-  const GT* __restrict__ gin = static_cast<const GT*>(a.g_in) + t.g_off;
-  const int* __restrict__ rest = a.rest_in + t.cell_off;
-  const int* __restrict__ pprev = a.p_prev + t.cell_off;
+  const GT* gin = static_cast<const GT*>(a.g_in) + t.g_off;
+  const int* rest = a.rest_in + t.cell_off;
+  const int* pprev = a.p_prev + t.cell_off;
   int* __restrict__ pcur = a.p_cur + t.cell_off;
   const int nxy = nx * ny;
   const bool ref = t.bc == kBcRef, walls = t.bc == kBcWallsZ;
@@ -370,14 +373,14 @@ __device__ __forceinline__ void phi_segment(const StepArgs& a, const Tile& t) {
       } else {
         const int xc = clampi(x, 1, nx - 2), yc = clampi(y, 1, ny - 2);
         const int zc = clampi(z, 1, nz - 2);
-        P = __ldg(pprev + xc + yc * nx + zc * nxy);
+        P = pprev[xc + yc * nx + zc * nxy];
       }
     } else {
       const int zm = (z == 0 ? nz - 1 : z - 1) * nxy;
       const int zp = (z == nz - 1 ? 0 : z + 1) * nxy;
       const bool blo = walls && z == 0, bhi = walls && z == nz - 1;
-      const int pself = S::kDev ? __ldg(pprev + idx) : 0;
-      P = S::rest_dec(__ldg(rest + idx), pself);
+      const int pself = S::kDev ? pprev[idx] : 0;
+      P = S::rest_dec(rest[idx], pself);
       static_for<1, kQ>([&](auto LC) {
         constexpr int L = decltype(LC)::value;
         constexpr int O = opp(L);
@@ -387,7 +390,7 @@ __device__ __forceinline__ void phi_segment(const StepArgs& a, const Tile& t) {
         } else {
           const int s = src_of<cz(L)>(zm, zo, zp) + src_of<cy(L)>(ym, yo, yp) +
                         src_of<cx(L)>(xm, x, xp);
-          const int ps = S::kDev ? __ldg(pprev + s) : 0;
+          const int ps = S::kDev ? pprev[s] : 0;
           P += S::template g_dec<L>(S::gload(gin + (L - 1) * n + s), ps);
         }
       });
@@ -448,8 +451,8 @@ __device__ __forceinline__ void phi_eq_segment(const StepArgs& a, const Tile& t)
   const int x = t.xt + static_cast<int>(threadIdx.x);
   const int y = t.yt + static_cast<int>(threadIdx.y);
   if (x >= nx || y >= ny) return;
-  const float4* __restrict__ rec = static_cast<const float4*>(a.j) + t.cell_off;
-  const int* __restrict__ pprev = a.p_prev + t.cell_off;
+  const float4* rec = static_cast<const float4*>(a.j) + t.cell_off;
+  const int* pprev = a.p_prev + t.cell_off;
   int* __restrict__ pcur = a.p_cur + t.cell_off;
   const int nxy = nx * ny;
   const bool ref = t.bc == kBcRef, walls = t.bc == kBcWallsZ;
@@ -465,12 +468,12 @@ __device__ __forceinline__ void phi_eq_segment(const StepArgs& a, const Tile& t)
       // Shell: zero-gradient copy of the previous update's interior phi.
       const int xc = clampi(x, 1, nx - 2), yc = clampi(y, 1, ny - 2);
       const int zc = clampi(z, 1, nz - 2);
-      return __ldg(pprev + xc + yc * nx + zc * nxy);
+      return pprev[xc + yc * nx + zc * nxy];
     }
     const int zm = (z == 0 ? nz - 1 : z - 1) * nxy;
     const int zp = (z == nz - 1 ? 0 : z + 1) * nxy;
     const bool blo = walls && z == 0, bhi = walls && z == nz - 1;
-    const float4 r0 = __ldg(rec + idx);
+    const float4 r0 = rec[idx];
     int P = wsplit_rest(__float_as_int(r0.x));
     auto pull = [&](auto LC) {
       constexpr int L = decltype(LC)::value;
@@ -481,7 +484,7 @@ __device__ __forceinline__ void phi_eq_segment(const StepArgs& a, const Tile& t)
       } else {
         const int src = src_of<cz(L)>(zm, zo, zp) + src_of<cy(L)>(ym, yo, yp) +
                         src_of<cx(L)>(xm, x, xp);
-        P += q_rec<L>(__ldg(rec + src));
+        P += q_rec<L>(rec[src]);
       }
     };
     // Nine records in flight at a time: the compiler may not hoist the second half of the
@@ -658,7 +661,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
   const float gravity = __ldg(&cd->gravity), phi_mean = __ldg(&cd->phi_mean);
   const float rho_out = kRatio ? __ldg(&cd->rho_out) : 1.f, drho = kRatio ? __ldg(&cd->drho) : 0.f;
 
-  const int* __restrict__ pcur = a.p_cur + t.cell_off;
+  const int* pcur = a.p_cur + t.cell_off;
 
   // Halo cells of a phi plane handled by this thread: their in-plane offsets are fixed.
   int hoff[KPF];
@@ -686,7 +689,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
     const int* base = pcur + static_cast<long long>(zmap(zpl)) * nxy;
 #pragma unroll
     for (int k = 0; k < KPF; ++k)
-      if (tid + k * NT < PP) pre[k] = __ldg(base + hoff[k]);
+      if (tid + k * NT < PP) pre[k] = base[hoff[k]];
   };
   auto commit = [&](int zpl) {
     float* d = sphi[(zpl + 5) % 5];
@@ -806,7 +809,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
   const int yp = (y == ny - 1 ? 0 : y + 1) * nx;
   const bool shell_xy = ref && (x == 0 || x == nx - 1 || y == 0 || y == ny - 1);
 
-  const FT* __restrict__ fin = static_cast<const FT*>(a.f_in) + t.f_off;
+  const FT* fin = static_cast<const FT*>(a.f_in) + t.f_off;
   FT* __restrict__ fout = static_cast<FT*>(a.f_out) + t.f_off;
   // f layout. Blocked (equilibrium g, all but the TMA kernel): population l of cell
   // (x, y, z) at fz(z) + fy(y) + fx(x) + l*32, with fz = z*PS, fy = y*RS,
@@ -823,12 +826,12 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
   const IT fy0 = kBlocked ? static_cast<IT>(y) * RS : 0;
   const IT fym = kBlocked ? static_cast<IT>(y == 0 ? ny - 1 : y - 1) * RS : 0;
   const IT fyp = kBlocked ? static_cast<IT>(y == ny - 1 ? 0 : y + 1) * RS : 0;
-  const GT* __restrict__ gin = static_cast<const GT*>(a.g_in) + t.g_off;
+  const GT* gin = static_cast<const GT*>(a.g_in) + t.g_off;
   GT* __restrict__ gout = static_cast<GT*>(a.g_out) + t.g_off;
-  const int* __restrict__ rest_in = (EQ || kPush) ? nullptr : a.rest_in + t.cell_off;
+  const int* rest_in = (EQ || kPush) ? nullptr : a.rest_in + t.cell_off;
   int* __restrict__ rest_out = (EQ || kPush) ? nullptr : a.rest_out + t.cell_off;
   float4* __restrict__ jout = EQ ? static_cast<float4*>(a.j) + t.cell_off : nullptr;
-  const int* __restrict__ pprev = a.p_prev + t.cell_off;
+  const int* pprev = a.p_prev + t.cell_off;
 
   // 16-bit relaxed g decodes every pulled population against the weight split of its source
   // cell's previous phi. A 4-plane ring of that previous phi (tile + halo 1, exact integers)
@@ -857,7 +860,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
       const int* base = pprev + static_cast<long long>(zq) * nxy;
 #pragma unroll
       for (int k = 0; k < KPR; ++k)
-        if ((k + 1) * NT <= HP || tid + k * NT < HP) ppre[k] = __ldg(base + proff[k]);
+        if ((k + 1) * NT <= HP || tid + k * NT < HP) ppre[k] = base[proff[k]];
     }
   };
   auto prev_commit = [&](int q) {
@@ -986,7 +989,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
     const bool blo = walls && z == 0, bhi = walls && z == nz - 1;
 
     // This cell's phi (read now, used after the barrier).
-    const int pc = active ? __ldg(pcur + idx) : 0;
+    const int pc = active ? pcur[idx] : 0;
     // Pull the 19 f populations (issued before the barriers to overlap their latency).
     FT fr[QF];
     if constexpr (kTma) {
@@ -1026,7 +1029,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
     } else if (work) {
       const IT fz0 = static_cast<IT>(z) * PS;
       // this cell's population 0
-      const FT* __restrict__ fc = kBlocked ? fin + (fz0 + fy0 + fx0) : fin + idx;
+      const FT* fc = kBlocked ? fin + (fz0 + fy0 + fx0) : fin + idx;
       // the stride between populations
       constexpr int kLS = kBlocked ? 32 : 0;
       const IT ls = kBlocked ? static_cast<IT>(kLS) : n;
@@ -1079,8 +1082,8 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
       if constexpr (kPush) {
         // no flux; the shell's own next phi is the lagged copy of its nearest interior cell
         push(z, pc, JQ{0, 0, 0});
-        pnext[idx] = __ldg(pcur + clampi(x, 1, nx - 2) + clampi(y, 1, ny - 2) * nx +
-                           clampi(z, 1, nz - 2) * nxy);
+        pnext[idx] = pcur[clampi(x, 1, nx - 2) + clampi(y, 1, ny - 2) * nx +
+                          clampi(z, 1, nz - 2) * nxy];
       } else if constexpr (EQ) {
         jout[idx] = make_float4(__int_as_float(pc), __int_as_float(0), __int_as_float(0),
                                 __int_as_float(0));
@@ -1305,7 +1308,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
       const int hcp = (ty + 1) * HX + tx + 1;  // this cell in the previous-phi ring
       int pself = 0;
       if constexpr (kPRing) pself = sprev[z & 3][hcp];
-      else if constexpr (S::kDev) pself = __ldg(pprev + idx);
+      else if constexpr (S::kDev) pself = pprev[idx];
       static_for<1, kQ>([&](auto LC) {
         constexpr int L = decltype(LC)::value;
         constexpr int O = opp(L);
@@ -1318,7 +1321,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
                         src_of<cx(L)>(xm, x, xp);
           int ps = 0;  // the source x - c_l: plane z - cz, row ty - cy, column tx - cx
           if constexpr (kPRing) ps = sprev[(z - cz(L)) & 3][hcp - cy(L) * HX - cx(L)];
-          else if constexpr (S::kDev) ps = __ldg(pprev + s);
+          else if constexpr (S::kDev) ps = pprev[s];
           gi = S::template g_dec<L>(S::gload(gin + (L - 1) * ng + s), ps);
         }
         const float gf = __int2float_rn(gi) * kInvQ30;

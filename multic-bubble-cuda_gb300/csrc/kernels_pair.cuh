@@ -90,6 +90,16 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
+// Two neighbouring 16-bit values with one 32-bit load.
+template <class T2>
+__device__ __forceinline__ T2 load_word(const void* p) {
+  static_assert(sizeof(T2) == sizeof(unsigned));
+  const unsigned w = *static_cast<const unsigned*>(p);
+  T2 v;
+  memcpy(&v, &w, sizeof v);
+  return v;
+}
+
 // Pair loads and stores of the storage formats. Deviation storage (16-bit) returns the
 // stored f - W; the moments add the weights' moments.
 template <class S>
@@ -102,17 +112,17 @@ struct PairIO<mcb::StF32> {
   using R2 = float2;
   using R1 = float;
   static __device__ __forceinline__ R2 raw2(const float* p) {
-    return __ldg(reinterpret_cast<const float2*>(p));
+    return *reinterpret_cast<const float2*>(p);
   }
-  static __device__ __forceinline__ R1 raw1(const float* p) { return __ldg(p); }
+  static __device__ __forceinline__ R1 raw1(const float* p) { return *p; }
   static __device__ __forceinline__ float2 cvt2(R2 v) { return v; }
   static __device__ __forceinline__ float cvt1(R1 v) { return v; }
   static __device__ __forceinline__ R1 lo(R2 v) { return v.x; }
   static __device__ __forceinline__ R1 hi(R2 v) { return v.y; }
   static __device__ __forceinline__ float2 ld2(const float* p) {
-    return __ldg(reinterpret_cast<const float2*>(p));
+    return *reinterpret_cast<const float2*>(p);
   }
-  static __device__ __forceinline__ float ld1(const float* p) { return __ldg(p); }
+  static __device__ __forceinline__ float ld1(const float* p) { return *p; }
   static __device__ __forceinline__ void st2(float* p, float2 v) {
     *reinterpret_cast<float2*>(p) = v;
   }
@@ -123,17 +133,17 @@ struct PairIO<mcb::StH16> {
   using R2 = __half2;
   using R1 = __half;
   static __device__ __forceinline__ R2 raw2(const __half* p) {
-    return __ldg(reinterpret_cast<const __half2*>(p));
+    return load_word<__half2>(p);
   }
-  static __device__ __forceinline__ R1 raw1(const __half* p) { return __ldg(p); }
+  static __device__ __forceinline__ R1 raw1(const __half* p) { return *p; }
   static __device__ __forceinline__ float2 cvt2(R2 v) { return __half22float2(v); }
   static __device__ __forceinline__ float cvt1(R1 v) { return __half2float(v); }
   static __device__ __forceinline__ R1 lo(R2 v) { return __low2half(v); }
   static __device__ __forceinline__ R1 hi(R2 v) { return __high2half(v); }
   static __device__ __forceinline__ float2 ld2(const __half* p) {
-    return __half22float2(__ldg(reinterpret_cast<const __half2*>(p)));
+    return __half22float2(load_word<__half2>(p));
   }
-  static __device__ __forceinline__ float ld1(const __half* p) { return __half2float(__ldg(p)); }
+  static __device__ __forceinline__ float ld1(const __half* p) { return __half2float(*p); }
   static __device__ __forceinline__ void st2(__half* p, float2 v) {
     *reinterpret_cast<__half2*>(p) = __float22half2_rn(v);
   }
@@ -144,18 +154,18 @@ struct PairIO<mcb::StB16> {
   using R2 = __nv_bfloat162;
   using R1 = __nv_bfloat16;
   static __device__ __forceinline__ R2 raw2(const __nv_bfloat16* p) {
-    return __ldg(reinterpret_cast<const __nv_bfloat162*>(p));
+    return load_word<__nv_bfloat162>(p);
   }
-  static __device__ __forceinline__ R1 raw1(const __nv_bfloat16* p) { return __ldg(p); }
+  static __device__ __forceinline__ R1 raw1(const __nv_bfloat16* p) { return *p; }
   static __device__ __forceinline__ float2 cvt2(R2 v) { return __bfloat1622float2(v); }
   static __device__ __forceinline__ float cvt1(R1 v) { return __bfloat162float(v); }
   static __device__ __forceinline__ R1 lo(R2 v) { return __low2bfloat16(v); }
   static __device__ __forceinline__ R1 hi(R2 v) { return __high2bfloat16(v); }
   static __device__ __forceinline__ float2 ld2(const __nv_bfloat16* p) {
-    return __bfloat1622float2(__ldg(reinterpret_cast<const __nv_bfloat162*>(p)));
+    return __bfloat1622float2(load_word<__nv_bfloat162>(p));
   }
   static __device__ __forceinline__ float ld1(const __nv_bfloat16* p) {
-    return __bfloat162float(__ldg(p));
+    return __bfloat162float(*p);
   }
   static __device__ __forceinline__ void st2(__nv_bfloat16* p, float2 v) {
     *reinterpret_cast<__nv_bfloat162*>(p) = __float22bfloat162_rn(v);
@@ -171,9 +181,9 @@ struct GPairIO<mcb::StF32> {
   using R2 = int2;
   using R1 = int;
   static __device__ __forceinline__ R2 raw2(const int* p) {
-    return __ldg(reinterpret_cast<const int2*>(p));
+    return *reinterpret_cast<const int2*>(p);
   }
-  static __device__ __forceinline__ R1 raw1(const int* p) { return __ldg(p); }
+  static __device__ __forceinline__ R1 raw1(const int* p) { return *p; }
   static __device__ __forceinline__ R1 lo(R2 v) { return v.x; }
   static __device__ __forceinline__ R1 hi(R2 v) { return v.y; }
   static __device__ __forceinline__ void st2(int* p, int a, int b) {
@@ -186,9 +196,9 @@ struct GPairIO<mcb::StH16> {
   using R2 = __half2;
   using R1 = __half;
   static __device__ __forceinline__ R2 raw2(const __half* p) {
-    return __ldg(reinterpret_cast<const __half2*>(p));
+    return load_word<__half2>(p);
   }
-  static __device__ __forceinline__ R1 raw1(const __half* p) { return __ldg(p); }
+  static __device__ __forceinline__ R1 raw1(const __half* p) { return *p; }
   static __device__ __forceinline__ R1 lo(R2 v) { return __low2half(v); }
   static __device__ __forceinline__ R1 hi(R2 v) { return __high2half(v); }
   static __device__ __forceinline__ void st2(__half* p, __half a, __half b) {
@@ -201,9 +211,9 @@ struct GPairIO<mcb::StB16> {
   using R2 = __nv_bfloat162;
   using R1 = __nv_bfloat16;
   static __device__ __forceinline__ R2 raw2(const __nv_bfloat16* p) {
-    return __ldg(reinterpret_cast<const __nv_bfloat162*>(p));
+    return load_word<__nv_bfloat162>(p);
   }
-  static __device__ __forceinline__ R1 raw1(const __nv_bfloat16* p) { return __ldg(p); }
+  static __device__ __forceinline__ R1 raw1(const __nv_bfloat16* p) { return *p; }
   static __device__ __forceinline__ R1 lo(R2 v) { return __low2bfloat16(v); }
   static __device__ __forceinline__ R1 hi(R2 v) { return __high2bfloat16(v); }
   static __device__ __forceinline__ void st2(__nv_bfloat16* p, __nv_bfloat16 a,
@@ -304,7 +314,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
   const float gravity = kOne ? a.one.gravity : __ldg(&cd->gravity);
   const float phi_mean = __ldg(&cd->phi_mean);  // from the table: new fields change it
 
-  const int* __restrict__ pcur = a.p_cur + t.cell_off;
+  const int* pcur = a.p_cur + t.cell_off;
   int* __restrict__ pnext = a.p_next + t.cell_off;
   int* __restrict__ pzero = a.p_zero + t.cell_off;
 
@@ -339,7 +349,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
 #pragma unroll
     for (int k = 0; k < KP2; ++k)
       if ((k + 1) * NT <= PP2 || tid + k * NT < PP2)  // whole rounds need no test
-        pre[k] = __ldg(reinterpret_cast<const int2*>(base + hoff[k]));
+        pre[k] = *reinterpret_cast<const int2*>(base + hoff[k]);
   };
   auto commit = [&](int zpl) {
     float2* d = reinterpret_cast<float2*>(sphi[slot5(zpl + 5)]);
@@ -443,7 +453,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
 
   // Blocked f layout: population l of cell (x, y, z) at z*PS + y*RS + fx(x) + 32 l, with
   // fx(x) = (x / 32) * 19 * 32 + x % 32. x0 is even, so x0 and x0 + 1 share a 32-cell block.
-  const FT* __restrict__ fin = static_cast<const FT*>(a.f_in) + t.f_off;
+  const FT* fin = static_cast<const FT*>(a.f_in) + t.f_off;
   FT* __restrict__ fout = static_cast<FT*>(a.f_out) + t.f_off;
   const int RS = t.fxb * (QF * 32);
   const long long PS = static_cast<long long>(RS) * ny;
@@ -482,9 +492,9 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
     else return make_float2(IO::cvt1(r1a[L]), IO::cvt1(r1b[L]));
   };
   // Stored g.
-  const GT* __restrict__ gin = static_cast<const GT*>(a.g_in) + t.g_off;
+  const GT* gin = static_cast<const GT*>(a.g_in) + t.g_off;
   GT* __restrict__ gout = static_cast<GT*>(a.g_out) + t.g_off;
-  const int* __restrict__ pprev = a.p_prev + t.cell_off;
+  const int* pprev = a.p_prev + t.cell_off;
   const int ng = static_cast<int>(t.ncell);
   // Relaxed g pulls the 18 stored populations of its sources; the 16-bit form decodes each
   // against its source's previous phi. Both are staged in shared memory with asynchronous
@@ -550,7 +560,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
   // Gathers the 19 populations of both cells of plane z and their Q2.30 phi.
   auto gather = [&](int z, int2& pcv) {
     const bool blo = walls && z == 0, bhi = walls && z == nz - 1;
-    pcv = __ldg(reinterpret_cast<const int2*>(pcur + x0 + yo + z * nxy));
+    pcv = *reinterpret_cast<const int2*>(pcur + x0 + yo + z * nxy);
     // Plane bases (the same for the whole block) plus this thread's byte offsets in the
     // plane, fixed for the segment; the population index is an immediate.
     const char* pz0 = reinterpret_cast<const char*>(fin + static_cast<long long>(z) * PS);
@@ -853,7 +863,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
       if (bounce) {
         const typename GIO::R2 v = GIO::raw2(gin + (O - 1) * ng + idx);
         int2 ps = make_int2(0, 0);
-        if constexpr (S::kDev) ps = __ldg(reinterpret_cast<const int2*>(pprev + idx));
+        if constexpr (S::kDev) ps = *reinterpret_cast<const int2*>(pprev + idx);
         ia = S::template g_dec<O>(GIO::lo(v), ps.x);
         ib = S::template g_dec<O>(GIO::hi(v), ps.y);
       } else {
@@ -1040,8 +1050,8 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
       // The shell's own next phi is the lagged copy of its nearest interior cell
       // (boundaryConditions, src/lbm.cu:403-425).
       const int zc = clampi(z, 1, nz - 2) * nxy, yc = clampi(y, 1, ny - 2) * nx;
-      if (sh0) pnext[idx] = __ldg(pcur + clampi(x0, 1, nx - 2) + yc + zc);
-      if (sh1) pnext[idx + 1] = __ldg(pcur + clampi(x0 + 1, 1, nx - 2) + yc + zc);
+      if (sh0) pnext[idx] = pcur[clampi(x0, 1, nx - 2) + yc + zc];
+      if (sh1) pnext[idx + 1] = pcur[clampi(x0 + 1, 1, nx - 2) + yc + zc];
     }
 
     if (a.macros) {

@@ -168,7 +168,7 @@ struct Solver {
     int grid_phi = 0, grid_collide = 0;
     int table = 0;  // first entry of the group's case table in d_gcases
     int has_ref = 0, single = 0;  // StepArgs of the same names
-    int chain = 0, smem = 0;
+    int chain = 0, early = 0;
   };
   std::vector<Group> groups;
   bool grouped = false;  // groups set by the batch autotuner (else one group, rebuilt)
@@ -355,31 +355,37 @@ struct Solver {
     g.single = cases.size() == 1 && !g.balanced &&
                (g.kernel == mcb::kPairAs0 || mcb::is_pair_variant(g.variant)) &&
                gmode != mcb::kGBgk;
-    return chain_of(g, nsm, occ_col);
+    chain_of(g, nsm, occ_col);
+    return MCB_OK;
   }
 
   // Whether a group's collide kernel is chained to the one before it (it may start under that
-  // one's last blocks), and the shared memory that goes with it. Chained blocks take whatever
-  // slots are free while the kernel before them runs: a grid that leaves free a good part of
-  // the slots then crowds on some SMs (64^3 relaxed FP32, 256 blocks on 456 slots: 25.8 us
-  // against 20.8). So a grid below one wave is limited, by its shared memory, to the blocks
-  // per SM that it needs anyway; then no SM holds more than the even spread's most. us per
-  // update, chained against not: 32^3 FP32 5.65 / 6.98, 64^3 FP16 12.6 / 14.1, 64^3 relaxed
-  // FP32 19.7 / 20.8, 80^3 FP32 24.3 / 26.1, 96^3 FP32 33.1 / 35.5, 97x75x61 25.7 / 27.5,
-  // 128x128x256 FP32 120.4 / 121.9, 256^3 BF16 413 / 416. The pair kernel with stored g loses
-  // (128x128x256 165 us against 160) and is not chained, nor is a batch in fixed chunks (64
-  // FP16 cases of 32..96 cells: 849 us against 835).
-  int chain_of(Group& g, int nsm, int occ_col) {
-    g.chain = g.smem = 0;
-    if (!push || (mcb::is_pair_variant(g.variant) && gmode != mcb::kGEquil) ||
-        (g.members.size() > 1 && !g.balanced))
-      return MCB_OK;
-    const int per_sm = (g.grid_collide + nsm - 1) / nsm;
-    if (per_sm < occ_col)
-      MCB_CU(mcb::residency_smem(storage, g.kernel, gmode, qf, ratio, wide, g.has_ref, g.single,
-                                 per_sm, &g.smem));
-    g.chain = per_sm >= occ_col || g.smem > 0;
-    return MCB_OK;
+  // one's end), and from where on it lets the next one start (early: with the last planes of
+  // its blocks).
+  //
+  // An early block takes whatever slot is free while this kernel's blocks hold theirs. A grid
+  // of about a wave or more leaves none that matters, and gains: 128x128x256 FP32 120.9 us per
+  // update against 123.0 unchained, 256^3 BF16 413 / 416, 97x75x61 25.5 / 27.5, 96^3 FP32
+  // 30.4 / 32.2. Below a wave the early blocks crowd on some SMs (80^3 relaxed FP32, 300 blocks
+  // on 456 slots: 44.8 us against 40.8; 34x33x71, 150 blocks: 19.7 against 17.5), so the next
+  // kernel starts with the end of this one's blocks: 40.3 and 17.0; 64^3 FP32 14.1 / 14.7,
+  // relaxed 64^3 20.4 / 21.0, 48^3 9.8 / 10.3. Blocks of one plane each on one block per SM are
+  // short enough to gain all the same: 32^3 FP32 5.4 / 7.0, 24^3 5.3 / 6.7. Over 242 lattices of
+  // 20 to 100 cells and all forms no such grid came out slower than unchained.
+  //
+  // No limit on the blocks per SM (shared memory that only keeps others away) holds a grid's
+  // even spread here, which one handle alone would gain from (48^3 8.7 us, relaxed 64^3 19.5):
+  // it keeps the blocks of other streams away too. us per update and handle, four handles side
+  // by side, without / with such a limit: 32^3 2.2 / 4.7, 48^3 6.4 / 8.2, 64^3 9.4 / 12.1,
+  // relaxed 64^3 15.0 / 17.8.
+  //
+  // The pair kernel with stored g loses chained (128x128x256 165 us against 160) and is not,
+  // nor is a batch in fixed chunks (64 FP16 cases of 32..96 cells: 849 us against 835).
+  void chain_of(Group& g, int nsm, int occ_col) {
+    g.chain = push && (!mcb::is_pair_variant(g.variant) || gmode == mcb::kGEquil) &&
+              (g.members.size() == 1 || g.balanced);
+    g.early = g.grid_collide > (occ_col - 1) * nsm ||
+              (g.zchunk == 1 && g.grid_collide <= nsm);
   }
 
   // Rebuilds the work decomposition of every group (one group of every case with the
@@ -771,7 +777,7 @@ struct Solver {
     a.ncases = static_cast<int>(gr.members.size());
     a.has_ref = gr.has_ref;
     a.chain = gr.chain;
-    a.smem = gr.smem;
+    a.early = gr.early;
     a.single = gr.single;
     if (a.single) a.one = cases[0];
     a.ntiles = gr.ntiles;

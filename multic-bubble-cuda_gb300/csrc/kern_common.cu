@@ -30,14 +30,8 @@ cudaError_t occupancy_f16(int variant, int gmode, int qf, int ratio, int wide,
                           int* phi_blocks, int* collide_blocks);
 cudaError_t occupancy_bf16(int variant, int gmode, int qf, int ratio, int wide,
                           int* phi_blocks, int* collide_blocks);
-cudaError_t residency_smem_f32(int variant, int gmode, int qf, int ratio, int wide, int has_ref,
-                               int single, int per_sm, int* bytes);
 cudaError_t launch_init_f32(const InitArgs& a, int nx, int ny, int nz, cudaStream_t s);
-cudaError_t residency_smem_f16(int variant, int gmode, int qf, int ratio, int wide, int has_ref,
-                               int single, int per_sm, int* bytes);
 cudaError_t launch_init_f16(const InitArgs& a, int nx, int ny, int nz, cudaStream_t s);
-cudaError_t residency_smem_bf16(int variant, int gmode, int qf, int ratio, int wide, int has_ref,
-                               int single, int per_sm, int* bytes);
 cudaError_t launch_init_bf16(const InitArgs& a, int nx, int ny, int nz, cudaStream_t s);
 
 namespace {
@@ -301,19 +295,6 @@ cudaError_t occupancy(int storage, int variant, int gmode, int qf, int ratio, in
     case kStF32: return occupancy_f32(variant, gmode, qf, ratio, wide, phi_blocks, collide_blocks);
     case kStF16: return occupancy_f16(variant, gmode, qf, ratio, wide, phi_blocks, collide_blocks);
     case kStBF16: return occupancy_bf16(variant, gmode, qf, ratio, wide, phi_blocks, collide_blocks);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-cudaError_t residency_smem(int storage, int variant, int gmode, int qf, int ratio, int wide,
-                           int has_ref, int single, int per_sm, int* bytes) {
-  switch (storage) {
-    case kStF32:
-      return residency_smem_f32(variant, gmode, qf, ratio, wide, has_ref, single, per_sm, bytes);
-    case kStF16:
-      return residency_smem_f16(variant, gmode, qf, ratio, wide, has_ref, single, per_sm, bytes);
-    case kStBF16:
-      return residency_smem_bf16(variant, gmode, qf, ratio, wide, has_ref, single, per_sm, bytes);
     default: return cudaErrorInvalidValue;
   }
 }

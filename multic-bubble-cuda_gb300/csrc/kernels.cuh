@@ -182,9 +182,12 @@ __device__ __forceinline__ void l2_prefetch(const void* p) {
 }
 
 // Programmatic dependent launch of the collide kernels: a block lets the next update's kernel
-// be launched as soon as every block of this one has started, and waits for the previous
-// kernel (complete, its writes visible) before its first access to the lattice. The launch
-// and the set-up of the offsets then run under the previous update's last blocks.
+// be launched once every block of this one has reached its last plane (StepArgs::early) or its
+// end, and waits for the previous kernel (complete, its writes visible) before its first access
+// to the lattice. The launch, and with early the set-up of the offsets too, then run under the
+// previous update's last blocks. Not sooner: blocks that only wait hold slots that the blocks
+// of another stream could use (two handles of 128x128x256 cells: 114.3 us per update of each
+// where the next kernel may start with the first plane, 113.5 with the last).
 // So a block may be alive while the kernel before it still writes phi, f and g. The read-only
 // path (__ldg, const __restrict__) is for data that nothing writes during a kernel's life:
 // here the case table alone. Phi, f and g go by plain loads, which stay behind the wait.
@@ -977,6 +980,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
   __syncthreads();
 
   for (int z = t.zb; z < t.ze; ++z) {
+    if (kPush && a.early && z == t.ze - 1) grid_trigger();
     commit(z + 3);
     if (z + 4 <= t.ze + 1) issue(z + 4);
 
@@ -1385,7 +1389,6 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
 template <class S, int GM, int BX, int BY>
 __global__ void __launch_bounds__(BX * BY, kCollideWarpsPerSM * 32 / (BX * BY))
     k_collide(const StepArgs a) {
-  grid_trigger();
   for_each_segment<BX, BY, true>(a,
                                  [&](const Tile& t) { collide_segment<S, GM, BX, BY>(a, t); }, a.balanced != 0);
 }
@@ -1393,7 +1396,6 @@ __global__ void __launch_bounds__(BX * BY, kCollideWarpsPerSM * 32 / (BX * BY))
 // Cases of 2^31 / 19 cells or more: 64-bit f offsets, 32x8 tiles.
 template <class S, int GM>
 __global__ void __launch_bounds__(256, kCollideWarpsPerSM / 8) k_collide_wide(const StepArgs a) {
-  grid_trigger();
   for_each_segment<32, 8, true>(
       a, [&](const Tile& t) { collide_segment<S, GM, 32, 8, false, kQ, false, true>(a, t); }, a.balanced != 0);
 }
@@ -1431,7 +1433,6 @@ constexpr int collide27_blocks() {
 template <class S, int GM, bool kWide>
 __global__ void __launch_bounds__(256, collide27_blocks<S, GM, kWide>())
     k_collide27(const StepArgs a) {
-  grid_trigger();
   for_each_segment<32, 8, true>(
       a, [&](const Tile& t) { collide_segment<S, GM, 32, 8, false, kQ27, false, kWide>(a, t); }, a.balanced != 0);
 }
@@ -1440,7 +1441,6 @@ __global__ void __launch_bounds__(256, collide27_blocks<S, GM, kWide>())
 template <class S, int GM, int QF, bool kWide>
 __global__ void __launch_bounds__(256, QF == kQ27 ? 2 : kCollideWarpsPerSM / 8)
     k_collide_ratio(const StepArgs a) {
-  grid_trigger();
   for_each_segment<32, 8, true>(
       a, [&](const Tile& t) { collide_segment<S, GM, 32, 8, false, QF, true, kWide>(a, t); }, a.balanced != 0);
 }
@@ -1684,21 +1684,6 @@ cudaError_t prepare_tma_kernel() {
                               TmaBox<typename S::FT>::kSmem);
 }
 
-// Opts a kernel in to the largest dynamic shared memory a block of it may have: one value for
-// every caller, so that no handle lowers what another one needs.
-inline cudaError_t opt_in_smem(const void* fn, int* largest = nullptr) {
-  cudaFuncAttributes at;
-  int dev = 0, block_max = 0;
-  cudaError_t e = cudaFuncGetAttributes(&at, fn);
-  if (e == cudaSuccess) e = cudaGetDevice(&dev);
-  if (e == cudaSuccess)
-    e = cudaDeviceGetAttribute(&block_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (e != cudaSuccess) return e;
-  const int most = block_max - static_cast<int>(at.sharedSizeBytes);
-  if (largest) *largest = most;
-  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-}
-
 // Resident blocks per SM of the phi and collide kernels of a variant.
 template <class S>
 cudaError_t occupancy_of(int variant, int gmode, int qf, int ratio, int wide, int* phi_blocks,
@@ -1745,7 +1730,7 @@ cudaError_t occupancy_of(int variant, int gmode, int qf, int ratio, int wide, in
     // shared memory per block is set here.
     dyn = pair_dyn_smem<S>(gmode);
     if (dyn > 0) {
-      e = opt_in_smem(fc);
+      e = cudaFuncSetAttribute(fc, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
       if (e != cudaSuccess) return e;
     }
   }
@@ -1785,34 +1770,6 @@ const void* collide_fn(int variant, int gmode, int qf, bool ratio, bool wide, bo
   return collide_kernel_gm<S>(variant, gmode, block);
 }
 
-// Dynamic shared memory that keeps a launch of that kernel to per_sm blocks per SM (0: what
-// the kernel needs already does, or it cannot be met), and the kernel's opt-in for it.
-template <class S>
-cudaError_t residency_smem_of(int variant, int gmode, int qf, int ratio, int wide, int has_ref,
-                              int single, int per_sm, int* bytes) {
-  *bytes = 0;
-  if (variant == kTmaVariant) return cudaSuccess;
-  dim3 block;
-  int dyn = 0, dev = 0, sm_total = 0, reserved = 0, largest = 0;
-  const void* fn = collide_fn<S>(variant, gmode, qf, ratio != 0, wide != 0, has_ref != 0,
-                                 single != 0, &block, &dyn);
-  if (!fn) return cudaErrorInvalidValue;
-  cudaFuncAttributes at;
-  cudaError_t e = cudaFuncGetAttributes(&at, fn);
-  if (e == cudaSuccess) e = cudaGetDevice(&dev);
-  if (e == cudaSuccess)
-    e = cudaDeviceGetAttribute(&sm_total, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-  if (e == cudaSuccess)
-    e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
-  if (e == cudaSuccess) e = opt_in_smem(fn, &largest);
-  if (e != cudaSuccess) return e;
-  // Past a (per_sm + 1)-th of the SM, in whole kilobytes.
-  const int fixed = static_cast<int>(at.sharedSizeBytes);
-  const int want = (sm_total / (per_sm + 1) - reserved - fixed) / 1024 * 1024 + 1024;
-  if (want > dyn && want <= largest) *bytes = want;
-  return cudaSuccess;
-}
-
 // One storage format per translation unit, so the formats compile in parallel.
 #define MCB_STORAGE_LAUNCHERS(S, suffix)                                                   \
   cudaError_t launch_phi_##suffix(int variant, int gmode, const StepArgs& a,               \
@@ -1831,12 +1788,7 @@ cudaError_t residency_smem_of(int variant, int gmode, int qf, int ratio, int wid
                                    a.has_ref != 0, a.single != 0, &block, &dyn);           \
     const dim3 grid = a.single ? dim3(a.one.tiles_x, a.one.tiles_y, a.one.tiles_z)         \
                                : dim3(a.grid_collide);                                     \
-    return launch_collide_fn(fn, grid, block, a, s, a.smem > dyn ? a.smem : dyn);          \
-  }                                                                                        \
-  cudaError_t residency_smem_##suffix(int variant, int gmode, int qf, int ratio, int wide, \
-                                      int has_ref, int single, int per_sm, int* bytes) {   \
-    return residency_smem_of<S>(variant, gmode, qf, ratio, wide, has_ref, single, per_sm,  \
-                                bytes);                                                    \
+    return launch_collide_fn(fn, grid, block, a, s, dyn);                                  \
   }                                                                                        \
   cudaError_t prepare_tma_##suffix() { return prepare_tma_kernel<S>(); }                   \
   size_t tma_smem_##suffix() { return TmaBox<typename S::FT>::kSmem; }                     \

@@ -640,6 +640,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
   __syncthreads();
 
   for (int z = t.zb; z < t.ze; ++z) {
+    if (EQ && a.early && z == t.ze - 1) grid_trigger();
     commit(z + 3);
     if (z + 4 <= t.ze + 1) issue(z + 4);
 
@@ -1075,7 +1076,6 @@ template <class S, bool kRef, int kMinBlocks, bool kL2, int GM, bool kOne, bool 
 __global__ void __launch_bounds__(PairShape<GM, RC>::TX * PairShape<GM, RC>::BY, kMinBlocks)
     k_collide_pair(const __grid_constant__ StepArgs a) {
   constexpr int BX = 2 * PairShape<GM, RC>::TX, BY = PairShape<GM, RC>::BY;
-  grid_trigger();
   if constexpr (kOne) {
     collide_pair_segment<S, kRef, kL2, GM, true, RC>(a, single_tile<BX, BY>(a));
     return;

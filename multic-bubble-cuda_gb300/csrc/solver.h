@@ -76,7 +76,7 @@ struct StepArgs {
   int grid_phi;        // blocks of the phi kernel
   int grid_collide;    // blocks of the collide kernel
   int chain;           // 1: the collide kernel may start under the end of the one before it
-  int smem;            // dynamic shared memory that limits its blocks per SM (0: none needed)
+  int early;           // 1: the one after it may start under this one's last planes
   int* err;            // set to a nonzero code when a bounded wait of a kernel gives up
   int qf;              // velocity set of f: 19 or 27 (every case of a launch)
   int ratio;           // 1: the density-ratio model (every case of a launch)
@@ -180,9 +180,6 @@ size_t tma_smem_bytes(int storage);
 // Resident blocks per SM of the phi and collide kernels of a tile variant.
 cudaError_t occupancy(int storage, int variant, int gmode, int qf, int ratio, int wide,
                       int* phi_blocks, int* collide_blocks);
-// Dynamic shared memory that limits a collide launch to per_sm blocks per SM (0: none).
-cudaError_t residency_smem(int storage, int variant, int gmode, int qf, int ratio, int wide,
-                           int has_ref, int single, int per_sm, int* bytes);
 cudaError_t launch_init(int storage, const InitArgs& a, int nx, int ny, int nz,
                         cudaStream_t s);
 cudaError_t launch_diag(const DiagArgs& a, cudaStream_t s);

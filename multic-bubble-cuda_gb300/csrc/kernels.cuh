@@ -175,6 +175,14 @@ __device__ __forceinline__ T nbr_of(T m, T o, T p) {
 __device__ __forceinline__ int wrap1(int v, int n) {
   return v < 0 ? v + n : (v >= n ? v - n : v);
 }
+// Single-precision operations that the compiler neither fuses nor splits. collide_segment names
+// every fused multiply-add of its equilibrium path with them, because the pair kernel's RC form
+// has to round alike (left to the compiler, another version or -fmad=false moved the fields of
+// one and not of the other).
+__device__ __forceinline__ float fmad(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float prod(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float plus(float a, float b) { return __fadd_rn(a, b); }
+
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return min(max(v, lo), hi); }
 
 __device__ __forceinline__ void l2_prefetch(const void* p) {
@@ -1140,14 +1148,14 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
       if constexpr (cx(L) != 0) cn += cx(L) * pl[0][o];
       if constexpr (cy(L) != 0) cn += cy(L) * pl[1][o];
       if constexpr (cz(L) != 0) cn += cz(L) * pl[2][o];
-      kap -= w3 * cn;
+      kap = fmad(-w3, cn, kap);
     });
     const float phi = sphi[(z + 5) % 5][(ty + 2) * PX + tx + 2];
     const float mult = sigma * kap;
-    float Fx = mult * nc.x * nc.w;
-    float Fy = mult * nc.y * nc.w;
-    float Fz = mult * nc.z * nc.w;
-    if (gravity != 0.f) Fz += gravity * (phi - phi_mean);
+    float Fx = prod(prod(mult, nc.x), nc.w);
+    float Fy = prod(prod(mult, nc.y), nc.w);
+    float Fz = prod(prod(mult, nc.z), nc.w);
+    if (gravity != 0.f) Fz = fmad(gravity, phi - phi_mean, Fz);
 
     // Moments (momentiCalc, src/lbm.cu:133-225). The non-equilibrium second moment is
     // sum c c (f - feq + HeF). For the D3Q19 second-order equilibrium its equilibrium
@@ -1196,6 +1204,7 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
       });
     }
     float ux, uy, uz, pxx, pyy, pzz, pxy, pxz, pyz, inv_rp = 0.f, rp = 1.f;
+    auto dot_uF = [&] { return fmad(uz, Fz, fmad(ux, Fx, prod(uy, Fy))); };
     if constexpr (kRatio) {
       // DensityRatio: velocity-based pressure formulation (Zu and He 2013; Fakhari et al.
       // 2017) with rho = rho_out + drho phi and grad rho = drho grad phi, grad phi being
@@ -1222,23 +1231,29 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
       pxz = sxz - ux * uz;
       pyz = syz - uy * uz;
     } else {
-      const float inv_rho = 1.0f / rho;
-      ux = (jx + 0.5f * Fx) * inv_rho;
-      uy = (jy + 0.5f * Fy) * inv_rho;
-      uz = (jz + 0.5f * Fz) * inv_rho;
-      const float uF = ux * Fx + uy * Fy + uz * Fz;
-      const float h = 1.5f * uF;
-      pxx = sxx - rho * (1.0f / 3.0f + ux * ux) + ux * Fx - h * ux * ux;
-      pyy = syy - rho * (1.0f / 3.0f + uy * uy) + uy * Fy - h * uy * uy;
-      pzz = szz - rho * (1.0f / 3.0f + uz * uz) + uz * Fz - h * uz * uz;
-      pxy = sxy - rho * ux * uy + 0.5f * (ux * Fy + uy * Fx) - h * ux * uy;
-      pxz = sxz - rho * ux * uz + 0.5f * (ux * Fz + uz * Fx) - h * ux * uz;
-      pyz = syz - rho * uy * uz + 0.5f * (uy * Fz + uz * Fy) - h * uy * uz;
+      const float inv_rho = __frcp_rn(rho);
+      ux = prod(fmad(0.5f, Fx, jx), inv_rho);
+      uy = prod(fmad(0.5f, Fy, jy), inv_rho);
+      uz = prod(fmad(0.5f, Fz, jz), inv_rho);
+      const float nh = prod(-1.5f, dot_uF());  // -h
+      const float hx = prod(nh, ux), hy = prod(nh, uy), hz = prod(nh, uz);
+      // p_ab = s_ab - rho (d_ab / 3 + u_a u_b) + (u_a F_b + u_b F_a) / 2 - h u_a u_b
+      auto diag = [&](float u, float F, float hu, float t, float s) {  // t = 1 / 3 + u^2
+        return fmad(hu, u, fmad(u, F, fmad(-rho, t, s)));
+      };
+      auto off = [&](float ua, float Fa, float ub, float Fb, float hu, float s) {
+        return fmad(hu, ub, fmad(0.5f, fmad(ua, Fb, prod(ub, Fa)), fmad(prod(-rho, ua), ub, s)));
+      };
+      pxx = diag(ux, Fx, hx, fmad(ux, ux, 1.0f / 3.0f), sxx);
+      pyy = diag(uy, Fy, hy, plus(1.0f / 3.0f, prod(uy, uy)), syy);
+      pzz = diag(uz, Fz, hz, fmad(uz, uz, 1.0f / 3.0f), szz);
+      pxy = off(ux, Fx, uy, Fy, hx, sxy);
+      pxz = off(ux, Fx, uz, Fz, hx, sxz);
+      pyz = off(uy, Fy, uz, Fz, hy, syz);
     }
-    const float uF = ux * Fx + uy * Fy + uz * Fz;
-    const float u2 = ux * ux + uy * uy + uz * uz;
-    const float h = 1.5f * uF;
-    const float tr3 = (pxx + pyy + pzz) * (1.0f / 3.0f);
+    const float uF = dot_uF();
+    const float u2 = fmad(uz, uz, fmad(ux, ux, prod(uy, uy)));
+    const float tr3 = prod(pxx + pyy + pzz, 1.0f / 3.0f);
 
     // Regularized collision with He forcing (collisionFluid, src/lbm.cu:233-288):
     //   f*_l = feq_l + (1 - omega) W_l/(2 cs^4) Q_l:Pi + HeF_l
@@ -1248,21 +1263,21 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
     const float om = (1.0f - omega) * 4.5f;
     // Deviation storage writes f*_l - W_l: the -1 folds into the shared term of each pair.
     constexpr float fshift = kDevF ? -1.0f : 0.0f;
-    const float R = rho - h;
+    const float R = plus(rho, prod(-1.5f, uF));
     // DensityRatio: f*_l = W_l [p* + 3 c.u + 9/2 (c.u)^2 - 3/2 u^2 + 9/2 (1 - omega) Q_l:Pi
     //                          + (1 - omega/2) 3 c.F / rho].
-    const float base = kRatio ? rho - 1.5f * u2 : 1.0f - 1.5f * u2;
+    const float base = kRatio ? rho - 1.5f * u2 : fmad(-1.5f, u2, 1.0f);
     const float cf = kRatio ? (1.0f - 0.5f * omega) * 3.0f * inv_rp : 0.f;
     // g collision (collisionPhase, src/lbm.cu:290-329):
     //   geq_l = W_l [phi (1 + 3 c.u) + sharp_c phi (1 - phi) c.n]
     // tau_g = 1 takes g* = geq as the reference does; otherwise BGK with omega_g.
-    const float A = sharp_c * phi * (1.0f - phi);
-    const float phi3 = 3.0f * phi;
+    const float A = prod(prod(sharp_c, phi), 1.0f - phi);
+    const float phi3 = prod(3.0f, phi);
 
     float fo[QF];
     float go[kQ];
     if constexpr (kRatio) fo[0] = wfq<QF>(0) * (base - om * tr3);
-    else fo[0] = wfq<QF>(0) * (base * R - om * tr3 + fshift);
+    else fo[0] = prod(wfq<QF>(0), plus(fmad(base, R, -prod(om, tr3)), fshift));
     static_for<0, (QF - 1) / 2>([&](auto KC) {
       constexpr int L = 2 * decltype(KC)::value + 1;
       constexpr int O = L + 1;
@@ -1274,9 +1289,10 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
       if constexpr (cx(L) * cy(L) != 0) qp += (2 * cx(L) * cy(L)) * pxy;
       if constexpr (cx(L) * cz(L) != 0) qp += (2 * cx(L) * cz(L)) * pxz;
       if constexpr (cy(L) * cz(L) != 0) qp += (2 * cy(L) * cz(L)) * pyz;
-      const float q = om * qp + fshift;
-      const float e0 = base + 4.5f * cu * cu, e1 = 3.0f * cu;
+      const float q = fmad(om, qp, fshift);
+      const float e0 = fmad(prod(4.5f, cu), cu, base);
       if constexpr (kRatio) {
+        const float e1 = 3.0f * cu;
         const float fe = cf * cF;
         fo[L] = W * (e0 + q + (e1 + fe));
         fo[O] = W * (e0 + q - (e1 + fe));
@@ -1285,9 +1301,8 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
         // changed the rounding of the small non-equilibrium part enough to shift the D3Q27
         // shear-wave viscosity by 4 %; summing opposite pairs first in the moments moved
         // the 2000-update static bubble 1.4e-4 from the FP64 oracle (1.5 % faster).
-        const float rf = 1.5f * cF;
-        fo[L] = W * ((e0 + e1) * (R + rf) + q);
-        fo[O] = W * ((e0 - e1) * (R - rf) + q);
+        fo[L] = prod(W, fmad(fmad(3.0f, cu, e0), fmad(1.5f, cF, R), q));
+        fo[O] = prod(W, fmad(fmad(-3.0f, cu, e0), fmad(-1.5f, cF, R), q));
       }
       if constexpr (L < kQ) {
         constexpr float WG = wf(L);  // g is D3Q19
@@ -1351,7 +1366,8 @@ __device__ __forceinline__ void collide_segment(const StepArgs& a, const Tile& t
     }
     if constexpr (EQ) {
       // Equilibrium storage: the 18 populations are W_l (phi + c_l . J), J = 3 phi u + A n.
-      const JQ jq = jq_of(phi3 * ux + A * nc.x, phi3 * uy + A * nc.y, phi3 * uz + A * nc.z);
+      const JQ jq = jq_of(fmad(A, nc.x, prod(phi3, ux)), fmad(A, nc.y, prod(phi3, uy)),
+                          fmad(A, nc.z, prod(phi3, uz)));
       if constexpr (kPush) push(z, pc, jq);
       else
         jout[idx] = make_float4(__int_as_float(pc), __int_as_float(jq.x), __int_as_float(jq.y),

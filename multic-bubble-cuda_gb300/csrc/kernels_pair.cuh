@@ -22,7 +22,7 @@
 //     register holds them across the plane's barrier;
 //   - the per-plane and per-segment work (phi ring, offsets, loop) is shared by two cells.
 // Arithmetic and the exact integer push of phi are those of k_collide, so results agree with
-// it to FP32 rounding (the fused multiply-adds are placed explicitly here). Requires an even
+// it to FP32 rounding; the RC form below agrees bit for bit. Requires an even
 // nx in every case, so that a pair never straddles the lattice edge.
 #pragma once
 
@@ -37,6 +37,11 @@ __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) {
 // a - b, exactly rounded: b * (-1) is exact, so the fused operation rounds once.
 __device__ __forceinline__ float2 sub(float2 a, float2 b) {
   return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a);
+}
+// a + p for a rounded product p. The assembler may fuse a packed product into the packed add
+// that follows it, even where both name their rounding; a factor of one keeps it from that.
+__device__ __forceinline__ float2 add_product(float2 a, float2 p) {
+  return __ffma2_rn(p, make_float2(1.0f, 1.0f), a);
 }
 __device__ __forceinline__ float2 scale(float2 a, float c) { return __fmul2_rn(a, dup(c)); }
 // s * a + b for a compile-time sign s = +1 or -1.
@@ -262,11 +267,11 @@ __host__ __device__ constexpr int pair_bgk_smem() {
 // kOne: the launch holds one case in fixed chunks, described by the kernel's parameters: the
 // per-plane bases and bounds then come from uniform registers and constants (508 warp
 // instructions per 32 cells against 532 at FP16, 110.3 us against 112.7 on 128x128x256).
-// RC: rounds every step as the one-cell kernel (k_collide, as the compiler fuses its
-// expressions) does, on that kernel's 32 x 8-cell tile, so that tile variant 0 gives the same
-// fields, bit for bit, from either: the curvature neighbour by neighbour, the force as (sigma
-// kappa n) |grad phi|, and the fused multiply-adds of u.F, u^2, Pi, f* and J in the order
-// marked RC below (equilibrium g; measured where the host picks it).
+// RC: rounds every step as the one-cell kernel, on that kernel's 32 x 8-cell tile, so that tile
+// variant 0 gives the same fields, bit for bit, from either. Both name the fused multiply-adds in
+// their source, in the same order: the curvature neighbour by neighbour, the force as (sigma
+// kappa n) |grad phi|, and u.F, u^2, Pi, f* and J as under RC below (equilibrium g; measured
+// where the host picks it).
 // GM: how g crosses the update (kGEquil: pushed equilibrium populations, nothing stored;
 // kGPop: stored at full relaxation; kGBgk: stored, pulled and relaxed with tau_g != 1). The
 // stored forms run periodic and wall modes only (no reference shell) and need 18 * cells
@@ -798,20 +803,21 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
     if constexpr (RC) {
       const float2 hx = mul(nh, ux), hy = mul(nh, uy), hz = mul(nh, uz);
       const float2 rx = mul(nrho, ux), ry = mul(nrho, uy);
-      auto diag = [&](float2 u, float2 F, float2 h, float2 sv) {
-        return fma(h, u, fma(u, F, fma(nrho, add(dup(1.0f / 3.0f), mul(u, u)), sv)));
+      auto diag = [&](float2 u, float2 F, float2 h, float2 t, float2 sv) {  // t = 1 / 3 + u^2
+        return fma(h, u, fma(u, F, fma(nrho, t, sv)));
       };
       auto off = [&](float2 ua, float2 Fa, float2 ub, float2 Fb, float2 ra, float2 ha,
                      float2 sv) {
         return fma(ha, ub, fma(dup(0.5f), fma(ua, Fb, mul(ub, Fa)), fma(ra, ub, sv)));
       };
-      pxx = diag(ux, Fx, hx, sxx);
-      pyy = diag(uy, Fy, hy, syy);
-      pzz = diag(uz, Fz, hz, szz);
+      const float2 third = dup(1.0f / 3.0f), uyy = mul(uy, uy);
+      pxx = diag(ux, Fx, hx, fma(ux, ux, third), sxx);
+      pyy = diag(uy, Fy, hy, pk::add_product(third, uyy), syy);
+      pzz = diag(uz, Fz, hz, fma(uz, uz, third), szz);
       pxy = off(ux, Fx, uy, Fy, rx, hx, sxy);
       pxz = off(ux, Fx, uz, Fz, rx, hx, sxz);
       pyz = off(uy, Fy, uz, Fz, ry, hy, syz);
-      u2 = fma(uz, uz, fma(ux, ux, mul(uy, uy)));
+      u2 = fma(uz, uz, fma(ux, ux, uyy));
     } else {
       const float2 uxx = mul(ux, ux), uyy = mul(uy, uy), uzz = mul(uz, uz);
       const float2 uxy = mul(ux, uy), uxz = mul(ux, uz), uyz = mul(uy, uz);
@@ -898,7 +904,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
     };
     const float2 om = dup((1.0f - omega) * 4.5f);
     constexpr float fshift = kDevF ? -1.0f : 0.0f;
-    const float2 R = add(rho, nh);
+    const float2 R = pk::add_product(rho, nh);
     const float2 base = fma(dup(-1.5f), u2, dup(1.0f));
     FT* __restrict__ fo_base = fout + static_cast<long long>(z) * PS + fy0 + fx0;
     // The shell lanes keep the value the init wrote: f = W (0 in deviation form).

@@ -270,10 +270,14 @@ struct Solver {
     // The longest chunk within 1 % of the least time (fewer primed planes); for several cases
     // the chunk of least time itself.
     double least = time_of(1);
-    for (int zc = 2; zc <= nzmax; ++zc) least = std::min(least, time_of(zc));
-    int best = nzmax;
-    const double slack = g.members.size() > 1 ? 1.0 : 1.01;
-    while (time_of(best) > slack * least) --best;
+    int at = 1;  // the longest chunk of least time
+    for (int zc = 2; zc <= nzmax; ++zc)
+      if (const double t = time_of(zc); t <= least) {
+        least = t;
+        at = zc;
+      }
+    int best = g.members.size() > 1 ? at : nzmax;
+    while (best > at && time_of(best) > 1.01 * least) --best;
     // Chunks of equal length: the same number of blocks, the last one not shorter.
     if (g.members.size() == 1) {
       const int m = (nzmax + best - 1) / best;

@@ -250,7 +250,8 @@ int  mcb_last_step_ms(mcb_handle* h, float* ms);
 int  mcb_step_profiled(mcb_handle* h, int nsteps, float* total_ms, float* phi_ms,
                        float* collide_ms);
 
-/* Kernel tile variants: count and shape (threads in x and y per block). */
+/* Kernel tile variants: count and shape (cells in x and y per block; variants 5 and 6: that of
+ * equilibrium g and of g stored at full relaxation, 64x4; with relaxed g they run 32x8). */
 int  mcb_variant_count(void);
 int  mcb_variant_shape(int variant, int* bx, int* by);
 

@@ -58,10 +58,12 @@ int fail(int code, const char* fmt, ...) {
 constexpr int kMaxWaves = 16;
 constexpr int kMinCollidePlanes = 8;
 // Default split of a batch: balanced runs of one wave up to this many tile-planes per block,
-// fixed chunks above. 34 uneven FP16 cases of 24..58 cells (34 planes per block) take 123 us
-// per update balanced against 137 to 155 in fixed chunks, 37 of 24..50 cells 94 against 96 to
-// 124; 64 of 32..96 cells (230 planes per block) 842 against 809, because neighbouring columns
-// no longer march in step and share less of L2.
+// fixed chunks above. 34 uneven FP16 cases of 24..58 cells take 130 us per update balanced
+// against 145 to 170 in fixed chunks, 37 of 24..50 cells 102 against 118 to 142, 100 of 32^3 89
+// against 97 to 125. 64 of 32..96 cells (about 220 planes per block) take 691 against 657, 48 at
+// FP32 542 against 468, because neighbouring columns no longer march in step and share less of
+// L2. In between 16 cases of 40..96 gain (189 against 195 or more), 8 of 96^3 do not (192, and
+// 187 in chunks of 32), and 24 of 48..80, above the line, would (207 against 222).
 constexpr int kBatchBalancedPlanes = 64;
 
 size_t pop_bytes(int storage) { return storage == mcb::kStF32 ? 4 : 2; }
@@ -248,7 +250,8 @@ struct Solver {
   //   one plane per block; 128x128x256 stays at 37 planes (one wave of 448 blocks).
   // Several cases share one launch, their blocks end at different times and the last wave
   // blurs: there the whole work over W counts, and a chunk for the end (64 FP16 cases of 32..96
-  // cells: 24 planes, 809 us, the best of 4 to 96; 32 planes 810, 52 planes 826).
+  // cells: 24 planes, 657 us, and 700, 677, 656 and 663 in chunks of 12, 16, 32 and 48; 48 FP32
+  // cases 18 planes, 468 us, and 460 in chunks of 20).
   int default_chunk(const Group& g, long long wave, int per_sm) const {
     constexpr double kPrime = 3.0;
     int nzmax = 1;
@@ -353,9 +356,11 @@ struct Solver {
     g.has_ref = 0;
     for (int ci : g.members) g.has_ref = g.has_ref || cases[ci].bc == mcb::kBcRef;
     // One case in fixed chunks goes by the kernel's parameters where the pair kernel runs
-    // (the y and z limits of a grid hold every lattice: at most 65535 cells per axis). 128 x
-    // 128 x 256: 121.5 us against 123.0 at FP32, 110.3 against 112.7 at FP16; relaxed g stays
-    // with the table (FP16 268 us against 264).
+    // (the y and z limits of a grid hold every lattice: at most 65535 cells per axis). us per
+    // update, parameters against the table: 48^3 FP32 9.6 / 9.9, 64^3 13.7 / 14.1; 128x128x256
+    // FP16 109.7 / 112.2, BF16 110.1 / 111.4, but FP32 120.9 / 119.2 (121.5 / 123.0 while the
+    // kernels read f through the read-only path); 256^3 BF16 413 / 418. Relaxed g stays with
+    // the table (on its former 64x4-cell tile FP16 268 us against 264).
     g.single = cases.size() == 1 && !g.balanced &&
                (g.kernel == mcb::kPairAs0 || mcb::is_pair_variant(g.variant)) &&
                gmode != mcb::kGBgk;
@@ -384,7 +389,8 @@ struct Solver {
   // relaxed 64^3 15.0 / 17.8.
   //
   // The pair kernel with stored g loses chained (128x128x256 165 us against 160) and is not,
-  // nor is a batch in fixed chunks (64 FP16 cases of 32..96 cells: 849 us against 835).
+  // nor is a batch in fixed chunks, where it gives 1 % at most (64 FP16 cases of 32..96 cells
+  // 654 against 657, 48 FP32 cases 465.5 against 467.7).
   void chain_of(Group& g, int nsm, int occ_col) {
     g.chain = push && (!mcb::is_pair_variant(g.variant) || gmode == mcb::kGEquil) &&
               (g.members.size() == 1 || g.balanced);
@@ -534,8 +540,12 @@ struct Solver {
     // Where nx leaves the pair kernel's 64-cell-wide tiles emptier than 32-wide ones, variant
     // 0 stays: 96^3, equilibrium g, 30.2 us against 37.8 (FP32), 26.6 against 35.7 (FP16); 80^3
     // 23.0 against 29.0. 200x200x100 (tiles 78 % full, against 89 %) runs the pair kernel.
-    // Stored g takes the pair kernel from 64^3 (there 24.8 us against 25.9 relaxed at FP16,
-    // at 32^3 10.6 against 8.2); where the line lies between them, fields would change with it.
+    // Stored g takes the pair kernel from 64^3 (there 24.8 us against 24.7 relaxed at FP16, at
+    // 48^3 16.5 against 15.3, at 32^3 10.6 against 7.1).
+    // The x fill is that of 64-cell-wide tiles for relaxed g too, although its pair tile is 32
+    // cells wide and would gain where it fills (FP16 96^3 57.1 us against 65.2, 160^3 234 against
+    // 276; 80^3 46.1 against 47.1): the two kernels round relaxed g differently, so another line
+    // would change the fields that those lattices give by default. variant 6 asks for it.
     auto x_fill = [&](int w) {  // share of the tiles' thread columns that hold cells
       double c = 0, t = 0;
       for (auto& d : cases) {

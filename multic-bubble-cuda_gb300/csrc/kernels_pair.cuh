@@ -505,7 +505,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
   // against its source's previous phi. Both are staged in shared memory with asynchronous
   // copies one plane ahead, so that no register holds them across the plane's barrier:
   //   - g of plane z: per population and tile row, the source row's words (2 cells each)
-  //     from x = xt - 2 to xt + 64 (words 0 .. TX + 1), in two buffers (z & 1);
+  //     from x = xt - 2 to xt + 2 TX + 1 (words 0 .. TX + 1), in two buffers (z & 1);
   //   - previous phi: rows yt - 1 .. yt + BY of a plane, the same x range, in a ring of
   //     four planes (q & 3): planes z - 1 .. z + 1 are read while z + 2 arrives.
   // Element 2 tx + 2 - cx of a staged row is the source x0 - cx of the pair's first cell.

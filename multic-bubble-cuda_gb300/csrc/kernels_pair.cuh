@@ -280,6 +280,9 @@ template <class S, bool kRef, bool kL2, int GM, bool kOne, bool RC>
 __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Tile& t) {
   constexpr bool EQ = GM == kGEquil;
   constexpr bool BGK = GM == kGBgk;
+  // The 16-bit shell instance that reads the case table has no register left for a trigger in
+  // the plane loop (it spills): it lets the next update start before its last flush instead.
+  constexpr bool kLateTrigger = EQ && kRef && S::kDev && !kOne && !RC;
   using GIO = pk::GPairIO<S>;
   using GT = typename GIO::GT;
   using FT = typename S::FT;
@@ -645,7 +648,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
   __syncthreads();
 
   for (int z = t.zb; z < t.ze; ++z) {
-    if (EQ && a.early && z == t.ze - 1) grid_trigger();
+    if (EQ && !kLateTrigger && a.early && z == t.ze - 1) grid_trigger();
     commit(z + 3);
     if (z + 4 <= t.ze + 1) issue(z + 4);
 
@@ -1074,6 +1077,7 @@ __device__ __forceinline__ void collide_pair_segment(const StepArgs& a, const Ti
     }
   }
   // The last target planes of the run.
+  if (kLateTrigger && a.early) grid_trigger();
   __syncthreads();
   for (int q = max(t.ze - 2, t.zb - 1); q <= t.ze; ++q) flush(q);
 }

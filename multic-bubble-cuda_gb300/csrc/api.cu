@@ -361,20 +361,22 @@ struct Solver {
     // FP16 109.7 / 112.2, BF16 110.1 / 111.4, but FP32 120.9 / 119.2 (121.5 / 123.0 while the
     // kernels read f through the read-only path); 256^3 BF16 413 / 418. Relaxed g stays with
     // the table (on its former 64x4-cell tile FP16 268 us against 264).
-    // Reference mode from about a wave on loses with the parameters (192^3 FP16 196 / 192, BF16
-    // 196.6 / 191.0, 128x128x256 FP16 115.7 / 113.8, 64x64x256 35.1 / 35.0) and gains below
-    // (40^3 9.6 / 10.4, 64^3 13.7 / 14.3); FP32 is even (128x128x256 128.9 either way).
+    // 16-bit reference mode from about a wave on loses with the parameters (192^3 FP16 196 / 192,
+    // BF16 196.6 / 191.0, 128x128x256 FP16 115.7 / 113.8, 64x64x256 35.1 / 35.0) and gains below
+    // (40^3 9.6 / 10.4, 64^3 13.7 / 14.3). FP32 is even chained (128x128x256 128.9 either way) and
+    // gains launch by launch (133.6 / 135.7, 64x64x256 45.2 / 46.4).
     g.single = cases.size() == 1 && !g.balanced && gmode != mcb::kGBgk &&
                (g.kernel == mcb::kPairAs0 ||
                 (mcb::is_pair_variant(g.variant) &&
-                 !(g.has_ref && g.grid_collide > (occ_col - 1) * nsm)));
+                 !(g.has_ref && storage != MCB_STORE_F32 &&
+                   g.grid_collide > (occ_col - 1) * nsm)));
     chain_of(g, nsm, occ_col);
     return MCB_OK;
   }
 
   // Whether a group's collide kernel is chained to the one before it (it may start under that
-  // one's end), and from where on it lets the next one start (early: with the last planes of
-  // its blocks).
+  // one's end), and from where on it lets the next one start (early: with the last plane of
+  // each block, of its first column piece in balanced runs).
   //
   // An early block takes whatever slot is free while this kernel's blocks hold theirs. A grid
   // of about a wave or more leaves none that matters, and gains: 128x128x256 FP32 120.9 us per

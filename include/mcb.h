@@ -86,7 +86,9 @@ typedef struct mcb_config {
                            -w (w <= 16) balanced over w waves of resident blocks, each
                            block taking an equal run of planes; 0 = default (the equal
                            chunks that fill whole waves of resident blocks best; a batch
-                           of small cases: one balanced wave) */
+                           of small cases: one balanced wave). The default is the fastest
+                           for one handle alone; several small handles stepped side by
+                           side can gain with longer chunks (four of 48^3: 4) */
     int   use_graph;    /* 1 = replay updates from a CUDA graph, 0 = plain launches */
     int   g_mode;       /* how g crosses between updates:
                            MCB_G_AUTO: with tau_g = 1 every post-collision g population is

@@ -265,8 +265,8 @@ __host__ __device__ constexpr int pair_bgk_smem() {
 // compiled only into that instance, which also runs the other modes.
 // kL2: prefetch into L2 the f rows of plane z + 2 while plane z collides.
 // kOne: the launch holds one case in fixed chunks, described by the kernel's parameters: the
-// per-plane bases and bounds then come from uniform registers and constants (508 warp
-// instructions per 32 cells against 532 at FP16, 110.3 us against 112.7 on 128x128x256).
+// per-plane bases and bounds then come from uniform registers and constants (511 warp
+// instructions per 32 cells against 532 at FP16, 109.7 us against 112.2 on 128x128x256).
 // RC: rounds every step as the one-cell kernel, on that kernel's 32 x 8-cell tile, so that tile
 // variant 0 gives the same fields, bit for bit, from either. Both name the fused multiply-adds in
 // their source, in the same order: the curvature neighbour by neighbour, the force as (sigma
